@@ -98,6 +98,19 @@ struct DevM2LGroup {
     long long t8_off;         // this group's transfer values: [ndir][ncand][kMaxGroup]
 };
 
+// M2L on one vector: up to four boxes of one level that share a parent and the
+// union of their list-2 sources in the order the lists hold them.  A candidate
+// has, for each target, its offset id as a 16-bit word, -1 where it is not in
+// that target's list 2.
+constexpr int kM2LFamily = 4;
+constexpr int kM2LMinTasksPerSM = 12;  // warps a level should keep busy per SM
+constexpr long long kM2LMinPairDirs = 3000000;
+struct DevM2LFamily {
+    int tgt[kM2LFamily];      // target boxes
+    int ntgt, empty_mask;     // bit t: target t has an empty list 2
+    int cand0, ncand;         // candidate range
+};
+
 // A stored near-field block (the reference's storage: each interaction once)
 // and one tile of it; see NearBlock and NearTile in plan.hpp.
 struct DevNearBlock {
@@ -344,6 +357,7 @@ private:
     std::string build_m2l_groups(const Plan& plan);
     size_t m2l_item_capacity(int min_chunk) const;
     void build_m2l_items(int max_chunk);
+    std::string build_m2l_families(const Plan& plan);
     std::string ensure_graph(int prec, bool tr);
     std::string setup_tc(const Plan& plan);
     std::string build_transl_device(const Level& L, double2* t);
@@ -373,6 +387,10 @@ private:
     int4* m2l_items_ = nullptr;          // (level, box, first direction, count)
     int n_m2l_items_ = 0;
     int m2l_first_[kMaxLevels] = {}, m2l_count_[kMaxLevels] = {};  // items of each level
+    DevM2LFamily* m2l_fams_ = nullptr;   // sibling families, level by level
+    int2* m2l_fam_off_ = nullptr;        // [candidate]: four 16-bit offset ids
+    int* m2l_fam_src_ = nullptr;         // [candidate]: source box
+    int m2l_fam_first_[kMaxLevels] = {}, m2l_fam_count_[kMaxLevels] = {};
     std::vector<char> m2l_has_list_[kMaxLevels];  // box has a non-empty list 2
     std::vector<int> m2l_len_[kMaxLevels];         // per level and box: list-2 length
     // Launch shapes (defaults at setup; mlfma_autotune may change them).

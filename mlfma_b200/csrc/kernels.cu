@@ -248,6 +248,115 @@ void DeviceOp::build_m2l_items(int max_chunk) {
     if (!items.empty()) h2d_landed(m2l_items_, items.data(), sizeof(int4) * items.size());
 }
 
+// Sibling families of the one-vector M2L (k_m2l_group): the boxes of a level
+// that share a parent, and their candidate sources in list order.  Every
+// sibling's list 2 is the sequence (parent's neighbours, their children) less
+// its own neighbours (Node::buildInteractionList, src/fmm/node.cpp:61-84), so
+// walking that sequence once meets each list in its own order.
+//
+// A warp's task is a family and a run of directions.  With four targets per
+// family a pattern load serves about three pairs, but a level of few boxes then
+// leaves most warps of the GPU without a task, so families shrink to two targets
+// or one until there are kM2LMinTasksPerSM per SM (the r = 1.13 sphere's 56-box
+// level with 392 directions: families of four 20 us, of one 16 us).  A level of
+// fewer than kM2LMinPairDirs (pair, direction)s gets no families and keeps
+// k_m2l_staged: filling the blocks' transfer values (81 KB each) is then most of
+// the work, and the large blocks queue behind the near field's (600 dipoles,
+// 2.0M: whole product 44.4 us staged, 45.4 us by families; a 512-box level of
+// 8,192 dipoles, 21M: product 181 and 150 us).
+std::string DeviceOp::build_m2l_families(const Plan& plan) {
+    std::vector<DevM2LFamily> fams;
+    std::vector<short> off;
+    std::vector<int> src;
+    for (int l = lmin_; l <= lmax_; ++l) {
+        const Level& L = plan.levels[l];
+        const size_t first = fams.size();
+        m2l_fam_first_[l] = static_cast<int>(first);
+        m2l_fam_count_[l] = 0;
+        if (static_cast<long long>(L.m2l_src.size()) * L.ndir < kM2LMinPairDirs) continue;
+        std::vector<int> order(L.boxes.size());
+        for (size_t b = 0; b < order.size(); ++b) order[b] = static_cast<int>(b);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+            return plan.nodes[L.boxes[a]].parent < plan.nodes[L.boxes[b]].parent;
+        });
+        size_t most = kM2LFamily;
+        for (; most > 1; most /= 2) {
+            size_t nf = 0;
+            for (size_t i = 0, j; i < order.size(); i = j) {
+                for (j = i; j < order.size() && plan.nodes[L.boxes[order[j]]].parent == plan.nodes[L.boxes[order[i]]].parent;) ++j;
+                nf += (j - i + most - 1) / most;
+            }
+            if (nf * ((L.ndir + kM2LDirs - 1) / kM2LDirs) >= static_cast<size_t>(kM2LMinTasksPerSM) * sms_) break;
+        }
+        std::vector<long long> work;
+        for (size_t i = 0; i < order.size();) {
+            const int par = plan.nodes[L.boxes[order[i]]].parent;
+            size_t j = i;
+            while (j < order.size() && plan.nodes[L.boxes[order[j]]].parent == par) ++j;
+            // several families of one parent stand next to one another, so that
+            // neighbouring warps read the same patterns
+            const size_t nsib = j - i, nfam = (nsib + most - 1) / most, per = (nsib + nfam - 1) / nfam;
+            long long all = 0;
+            for (size_t q = i; q < j; ++q) all += L.m2l_ptr[order[q] + 1] - L.m2l_ptr[order[q]];
+            for (; i < j; i += std::min(per, j - i)) {
+                DevM2LFamily f{};
+                f.cand0 = static_cast<int>(src.size());
+                int at[kM2LFamily], len[kM2LFamily];
+                long long pairs = 0;
+                for (size_t q = i; q < std::min(i + per, j); ++q) {
+                    const int b = order[q], t = f.ntgt++;
+                    f.tgt[t] = b;
+                    at[t] = 0;
+                    len[t] = L.m2l_ptr[b + 1] - L.m2l_ptr[b];
+                    pairs += len[t];
+                    if (!len[t]) f.empty_mask |= 1 << t;
+                }
+                if (!pairs && ref_compat_) continue;  // nothing written (node.cpp:106-108)
+                long long met = 0;
+                for (int bn : plan.nodes[par].nbors)
+                    for (int c = 0; c < 8; ++c) {
+                        const int ch = plan.nodes[bn].child[c];
+                        const int box = ch < 0 ? -1 : plan.nodes[ch].box;
+                        if (box < 0) continue;
+                        short o[kM2LFamily];
+                        bool used = false;
+                        for (int t = 0; t < kM2LFamily; ++t) {
+                            o[t] = -1;
+                            if (t >= f.ntgt || at[t] >= len[t]) continue;
+                            const int p = L.m2l_ptr[f.tgt[t]] + at[t];
+                            if (L.m2l_src[p] != box) continue;
+                            o[t] = static_cast<short>(L.m2l_off[p]);
+                            ++at[t];
+                            ++met;
+                            used = true;
+                        }
+                        if (!used) continue;
+                        src.push_back(box);
+                        off.insert(off.end(), o, o + kM2LFamily);
+                    }
+                if (met != pairs) return "internal: interaction lists of siblings in different orders";
+                f.ncand = static_cast<int>(src.size()) - f.cand0;
+                fams.push_back(f);
+                work.push_back(all);
+            }
+        }
+        // largest families first (the last round short); families write their
+        // own boxes, so the order changes no result
+        std::vector<size_t> by(work.size());
+        for (size_t i = 0; i < by.size(); ++i) by[i] = i;
+        std::stable_sort(by.begin(), by.end(), [&](size_t a, size_t b) { return work[a] > work[b]; });
+        std::vector<DevM2LFamily> sorted(by.size());
+        for (size_t i = 0; i < by.size(); ++i) sorted[i] = fams[first + by[i]];
+        std::copy(sorted.begin(), sorted.end(), fams.begin() + first);
+        m2l_fam_count_[l] = static_cast<int>(fams.size() - first);
+    }
+    m2l_fams_ = upload(fams);
+    m2l_fam_src_ = upload(src);
+    m2l_fam_off_ = alloc<int2>(src.size());
+    if (!off.empty()) MLFMA_CK(h2d_landed(m2l_fam_off_, off.data(), off.size() * sizeof(short)));
+    return {};
+}
+
 // The 316 x ndir transfer functions of level L on the GPU (k_tables_alpha,
 // k_tables_transl), complex double, into t.
 std::string DeviceOp::build_transl_device(const Level& L, double2* t) {
@@ -457,6 +566,8 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         MLFMA_CK(cudaFuncSetAttribute(t ? k_l2l<R, 24, true> : k_l2l<R, 24, false>, attr, dev_smem));
         MLFMA_CK(cudaFuncSetAttribute(t ? k_l2l<R, 32, true> : k_l2l<R, 32, false>, attr, dev_smem));
         MLFMA_CK(cudaFuncSetAttribute(t ? k_s2m<R, true> : k_s2m<R, false>, attr, dev_smem));
+        if constexpr (std::is_same<R, double>::value)
+            MLFMA_CK(cudaFuncSetAttribute(t ? k_m2l_group<true> : k_m2l_group<false>, attr, dev_smem));
         if constexpr (!std::is_same<R, double>::value) {
             MLFMA_CK(cudaFuncSetAttribute(t ? k_s2m_half<R, true> : k_s2m_half<R, false>, attr, dev_smem));
             MLFMA_CK(cudaFuncSetAttribute(t ? k_l2t_half<R, true> : k_l2t_half<R, false>, attr, dev_smem));
@@ -609,6 +720,11 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
         }
         m2l_items_ = alloc<int4>(m2l_item_capacity(8));
         build_m2l_items(128);
+        MLFMA_CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
+        {
+            const std::string e = build_m2l_families(plan);
+            if (!e.empty()) return e;
+        }
 
         // ---- transitions: L2L pairs and stencil widths
         l2l_pairs_.assign(std::max(lmax_, 0) + 1, nullptr);
@@ -789,7 +905,6 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
                 MLFMA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&near_direct_occ_, k_near_direct, kNdThreads, 0));
                 near_direct_occ_ = std::max(1, near_direct_occ_);
                 near_per_sm_ = near_occ_;
-                MLFMA_CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
                 set_near_grid(near_per_sm_);
                 DevNearBlock* d_nb = upload(nb);
                 k_near_blocks_assemble<<<blocks_for(near_block_entries_, 128), 128, 0, stream_>>>(
@@ -921,6 +1036,31 @@ void DeviceOp::far_m2l(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl)
     const int first = m2l_first_[lo];
     const int count = m2l_first_[hi] + m2l_count_[hi] - first;
     if (count <= 0) return;
+    if constexpr (std::is_same<R, double>::value) {
+        if (m2l_staged_) {
+            for (int l = lo; l <= hi; ++l) {
+                const int nf = m2l_fam_count_[l];
+                if (!nf) {  // a level below the families' threshold
+                    if (m2l_count_[l])
+                        launch_k(pdl, k_m2l_staged<R, TR>, m2l_count_[l], 128, 0, s, F.lv_dev,
+                                 m2l_items_ + m2l_first_[l], ref_compat_ ? 0 : 1);
+                    pdl = pdl && !m2l_count_[l];
+                    continue;
+                }
+                // Every block fills its transfer values once and then streams
+                // families: as many warps share a block as the level keeps
+                // busy, and one wave of blocks, two to an SM.
+                const int nchunk = (ndir_[l] + kM2LDirs - 1) / kM2LDirs;
+                const long long tasks = static_cast<long long>(nf) * nchunk;
+                const int warps = static_cast<int>(std::max(1ll, std::min<long long>(kM2LMaxWarps, tasks / (2 * sms_))));
+                const int nsplit = std::max(1, std::min((nf + warps - 1) / warps, 2 * sms_ / nchunk));
+                launch_k(pdl, k_m2l_group<TR>, nchunk * nsplit, 32 * warps, m2l_group_smem(warps), s, F.lv_dev, l,
+                         m2l_fams_ + m2l_fam_first_[l], nf, m2l_fam_off_, m2l_fam_src_, nchunk, ref_compat_ ? 0 : 1);
+                pdl = false;  // the levels of one call do not depend on one another
+            }
+            return;
+        }
+    }
     launch_k(pdl, m2l_staged_ ? k_m2l_staged<R, TR> : k_m2l<R, TR>, count, 128, 0, s, F.lv_dev, m2l_items_ + first,
              ref_compat_ ? 0 : 1);
 }

@@ -9,6 +9,8 @@
 // pattern is one contiguous run of 2*ndir values.
 #pragma once
 
+#include <type_traits>
+
 #include "device.cuh"
 #include "zmath.cuh"
 #include "bulk_copy.cuh"
@@ -518,6 +520,154 @@ k_m2l_staged(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ item
     const R w = lv.w[d];
     Bo[0] = cscale(w, cadd(a0, c0));
     Bo[1] = cscale(w, cadd(a1, c1));
+}
+
+// The complex-double translation for up to four boxes of one parent together.
+// Siblings share most of their candidate sources (the children of the parent's
+// neighbours), so a warp takes one family of siblings and 16 directions (lane =
+// (direction, component)), keeps the targets' sums in registers, loads every
+// candidate's pattern once for all of them, and reads the transfer values from
+// shared memory, where the block holds all 316 offsets of its directions: per
+// (pair, direction) one 16-byte shared-memory read and a fraction of a pattern
+// load, in place of a transfer value and a whole pattern from L2.  Block = (run
+// of directions, every nsplit-th batch of the level's families); each warp has
+// its next family's header and the next 32 candidates in flight while it
+// computes, and four or eight patterns ahead.
+//
+// Bound by shared-memory reads (two wavefronts a pair, four a pattern) and
+// instruction issue, so a candidate's transfer rows are staged as shared-memory
+// offsets (a row of zeros where it is not in a target's list 2, about one pair
+// in ten) and the loop is instantiated per number of targets: a shared-memory
+// read and four multiply-adds per pair.  (A source value that is not finite
+// reaches every target anyhow, by a list or through the near field, so the zero
+// rows spread nothing.)  One B200, k_m2l_staged -> this: 8,192 dipoles, level 3
+// (512 boxes, 392 directions) 77 -> 46 us; r = 8 sphere, level 6 (16,344 boxes,
+// 162 directions) 390 -> 204 us, all levels 930 -> 530 us; r = 2 sphere,
+// levels 2-4 22/28/34 -> 20/22/27 us.  In complex float, whose sums keep
+// their order and run in two halves, the same form was issue-bound and no
+// faster (r = 2 sphere 18/19/22 -> 20/26/34 us, r = 8 sphere 498 -> 505 us):
+// complex float keeps k_m2l_staged.
+constexpr int kM2LOffsets = 316;
+constexpr int kM2LDirs = 16;            // directions per block
+constexpr int kM2LRow = kM2LDirs * 16;  // bytes of a row of transfer values
+constexpr int kM2LMaxWarps = 12;        // two blocks per SM at 80 registers
+constexpr int kM2LPerWarp = 32 * (sizeof(int4) + sizeof(int));  // staged candidates
+constexpr size_t m2l_group_smem(int warps) {
+    return static_cast<size_t>(kM2LOffsets + 1) * kM2LRow + static_cast<size_t>(warps) * kM2LPerWarp;
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+template <bool TR>
+__global__ void __launch_bounds__(32 * kM2LMaxWarps, 2)
+k_m2l_group(const DevLevelT<double>* __restrict__ lvs, int level, const DevM2LFamily* __restrict__ fams, int nfam,
+            const int2* __restrict__ cand_off, const int* __restrict__ cand_src, int nchunk, int zero_empty) {
+    chain_wait();
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double2* tsm = reinterpret_cast<double2*>(smraw);  // [316 + 1][kM2LDirs], the last row zero
+    const int nwarp = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* cand = smraw + (kM2LOffsets + 1) * kM2LRow;
+    int4* soff = reinterpret_cast<int4*>(cand) + warp * 32;
+    int* ssrc = reinterpret_cast<int*>(cand + sizeof(int4) * 32 * nwarp) + warp * 32;
+    const DevLevelT<double> lv = lvs[level];
+    const int ndir = lv.ndir;
+    const int chunk = blockIdx.x % nchunk, split = blockIdx.x / nchunk, nsplit = gridDim.x / nchunk;
+    const int d0 = chunk * kM2LDirs, dn = min(kM2LDirs, ndir - d0);
+    for (int i = threadIdx.x; i < kM2LOffsets * kM2LDirs; i += blockDim.x) {
+        const int o = i / kM2LDirs, q = i - o * kM2LDirs;
+        if (q < dn) cp_async16(tsm + i, lv.transl + static_cast<size_t>(TR ? kM2LOffsets - 1 - o : o) * ndir + d0 + q);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (threadIdx.x < kM2LDirs) tsm[kM2LOffsets * kM2LDirs + threadIdx.x] = z0();
+    const int dl = min(lane >> 1, dn - 1), comp = lane & 1;
+    const bool live = (lane >> 1) < dn;
+    const int d = d0 + dl;
+    const double w = lv.w[d];
+    const unsigned char* tl = reinterpret_cast<const unsigned char*>(tsm + dl);
+    const double2* Al = lv.A + 2 * static_cast<size_t>(d) + comp;
+    const size_t astride = 2 * static_cast<size_t>(ndir);
+    // families largest first: neighbouring warps take families of one parent
+    // (two at a time), blocks take them in turn
+    const int step = nsplit * nwarp, nw2 = nwarp & ~1;
+    int f = warp < nw2 ? 2 * ((warp >> 1) * nsplit + split) + (warp & 1) : nw2 * nsplit + split;
+    const int* hdr = reinterpret_cast<const int*>(fams);
+    constexpr int HW = sizeof(DevM2LFamily) / sizeof(int);
+    static_assert(HW == 8 && kM2LFamily == 4, "a family header is one word per lane of a quarter warp");
+    int hv = f < nfam ? hdr[static_cast<size_t>(f) * HW + (lane & 7)] : 0;
+    int hn = 0;
+    int2 co = make_int2(-1, -1);
+    int cs = 0;
+    auto fetch = [&](int h, int c0) {  // this lane's candidate of the batch at c0
+        const int cand0 = __shfl_sync(0xffffffffu, h, 6), n = __shfl_sync(0xffffffffu, h, 7);
+        const int c = min(c0 + lane, n - 1);
+        co = make_int2(-1, -1);
+        cs = 0;
+        if (c >= 0) cs = cand_src[cand0 + c];
+        if (c0 + lane < n) co = cand_off[cand0 + c];
+    };
+    auto row = [](int o) { return (o < 0 ? kM2LOffsets : o) * kM2LRow; };
+    auto family = [&](auto nt) {  // one family of NT targets
+        constexpr int NT = decltype(nt)::value;
+        constexpr int U = NT > 2 ? 4 : 8;  // patterns loaded ahead
+        double2 acc[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = z0();
+        const int ncand = __shfl_sync(0xffffffffu, hv, 7);
+        for (int c0 = 0; c0 < ncand; c0 += 32) {
+            __syncwarp();
+            soff[lane] = make_int4(row(static_cast<short>(co.x & 0xffff)), row(co.x >> 16),
+                                   row(static_cast<short>(co.y & 0xffff)), row(co.y >> 16));
+            ssrc[lane] = cs;
+            __syncwarp();
+            if (c0 + 32 < ncand) fetch(hv, c0 + 32); else fetch(hn, 0);
+            const int nb = min(32, ncand - c0);
+            double2 a[U], an[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) a[u] = Al[ssrc[u] * astride];
+            for (int i = 0; i < nb; i += U) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) an[u] = Al[ssrc[(i + U + u) & 31] * astride];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int4 o4 = soff[i + u];  // (past the list's end: rows of zeros)
+                    const int o[4] = {o4.x, o4.y, o4.z, o4.w};
+                    double2 tv[NT];
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) tv[t] = *reinterpret_cast<const double2*>(tl + o[t]);
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) acc[t] = cfma(tv[t], a[u], acc[t]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) a[u] = an[u];
+            }
+        }
+        if (ncand == 0) fetch(hn, 0);
+        const int empty = __shfl_sync(0xffffffffu, hv, 5);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int box = __shfl_sync(0xffffffffu, hv, t);
+            const bool none = (empty >> t) & 1;
+            // (an empty list under the reference's rule: kept from the previous product)
+            if (live && (!none || zero_empty))
+                lv.B[(static_cast<size_t>(box) * ndir + d) * 2 + comp] = none ? z0() : cscale(w, acc[t]);
+        }
+    };
+    fetch(hv, 0);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the transfer values
+    for (; f < nfam; f += step) {
+        const int fn = f + step;
+        hn = fn < nfam ? hdr[static_cast<size_t>(fn) * HW + (lane & 7)] : 0;
+        switch (__shfl_sync(0xffffffffu, hv, 4)) {
+            case 1: family(std::integral_constant<int, 1>()); break;
+            case 2: family(std::integral_constant<int, 2>()); break;
+            case 3: family(std::integral_constant<int, 3>()); break;
+            default: family(std::integral_constant<int, 4>()); break;
+        }
+        hv = hn;
+    }
 }
 
 // ------------------------------------------------------------ L2L
