@@ -84,6 +84,24 @@ struct DevFarLeaf {
     long long pat_off;
 };
 
+// One work item of aggregation (a leaf and a run of at most a block's threads of
+// pattern elements) and of disaggregation (a leaf and a run of its sources),
+// with everything the kernel needs: a block's streaming loads wait for one load.
+template <class R>
+struct DevS2MItem {
+    const typename Cx<R>::T* pat;  // the leaf's first source, first element of the run
+    typename Cx<R>::T* a;          // the box's outgoing pattern
+    const int* anti;               // DevLevelT::anti of the leaf's level
+    int src0, nsrc, ne, e0, ec, pad;
+};
+template <class R>
+struct DevL2TItem {
+    const typename Cx<R>::T* pat;  // the run's first source
+    const typename Cx<R>::T* b;    // the box's local pattern
+    const int* anti;
+    int src0, cnt, ne, pad;
+};
+
 // M2L on many right-hand sides: the boxes of one level that share a parent
 // (at most 8) and the union of their list-2 sources; for each candidate source
 // the offset id towards every target (-1: not in that target's list 2).
@@ -206,6 +224,8 @@ struct FarField {
     std::vector<DevTransT<R>> trans;  // index = parent level
     C* pat = nullptr;                 // radiation patterns [pat_elems][2] (FP64; many right-hand sides)
     C* hpat = nullptr;                // complex float: directions d < ndir/2 of each source, [pat_elems / 2][2]
+    DevS2MItem<R>* s2m = nullptr;     // work items (counts: DeviceOp::n_s2m_items_, n_l2t_items_)
+    DevL2TItem<R>* l2t = nullptr;
     C* m2l_t8 = nullptr;              // many-rhs M2L: pre-gathered weighted transfer values
 };
 
@@ -408,12 +428,9 @@ private:
     int m_l2l_pairs_ = 0;                 // many-rhs L2L column pairs per block (0: precision default)
     std::vector<int2*> l2l_pairs_;       // per parent level: (parent, child entry)
     std::vector<int> n_l2l_pairs_, npar_, up_w_, dn_w_;
-    int4* s2m_items_ = nullptr;          // (leaf, first element, element count)
-    int n_s2m_items_ = 0;
-    int4* s2m_items_h_ = nullptr;        // the same over the stored half (half patterns)
-    int n_s2m_items_h_ = 0;
-    int4* l2t_items_ = nullptr;          // (leaf, first source, source count)
-    int n_l2t_items_ = 0;
+    std::vector<int4> s2m_items_[2];     // per precision: (leaf, first element, element count)
+    std::vector<int4> l2t_items_;        // (leaf, first source, source count)
+    int n_s2m_items_[2] = {}, n_l2t_items_ = 0;
     int max_src_ = 0;                    // largest far leaf
     int max_leaf_ndir_ = 0;              // most directions on a level holding far leaves
     bool far_covers_all_ = false;        // every source sits in a far leaf (L2T writes all of yfar_)

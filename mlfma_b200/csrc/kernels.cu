@@ -532,6 +532,27 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         if (n_leaves_) k_half_patterns<R><<<n_leaves_, 256, 0, stream_>>>(F.lv_dev, leaves_, pat64, F.hpat);
         MLFMA_CK(cudaGetLastError());
     }
+    {  // work items of aggregation and disaggregation
+        constexpr bool f64 = std::is_same<R, double>::value;
+        const C* pat = f64 ? F.pat : F.hpat;
+        const int per_dir = f64 ? 2 : 1;  // stored values per direction
+        std::vector<DevS2MItem<R>> up;
+        for (const int4& q : s2m_items_[f64 ? kFp64 : kMixed]) {
+            const FarLeaf& f = plan.far_leaves[q.x];
+            const DevLevelT<R>& d = F.lv[f.level];
+            up.push_back({pat + f.pat_off * per_dir + q.y, d.A + static_cast<size_t>(f.box) * d.ndir * 2, d.anti, f.src0,
+                          f.nsrc, d.ndir * per_dir, q.y, q.z, 0});
+        }
+        std::vector<DevL2TItem<R>> dn;
+        for (const int4& q : l2t_items_) {
+            const FarLeaf& f = plan.far_leaves[q.x];
+            const DevLevelT<R>& d = F.lv[f.level];
+            dn.push_back({pat + (f.pat_off + static_cast<long long>(q.y) * d.ndir) * per_dir,
+                          d.B + static_cast<size_t>(f.box) * d.ndir * 2, d.anti, f.src0 + q.y, q.z, d.ndir * per_dir, 0});
+        }
+        F.s2m = upload(up);
+        F.l2t = upload(dn);
+    }
     // Shared-memory limits.
     size_t m2m_smem = 1, l2l_smem = 1;
     for (int p = lmin_; p < lmax_; ++p) {
@@ -565,9 +586,11 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         MLFMA_CK(cudaFuncSetAttribute(t ? k_l2l<R, 16, true> : k_l2l<R, 16, false>, attr, dev_smem));
         MLFMA_CK(cudaFuncSetAttribute(t ? k_l2l<R, 24, true> : k_l2l<R, 24, false>, attr, dev_smem));
         MLFMA_CK(cudaFuncSetAttribute(t ? k_l2l<R, 32, true> : k_l2l<R, 32, false>, attr, dev_smem));
-        MLFMA_CK(cudaFuncSetAttribute(t ? k_s2m<R, true> : k_s2m<R, false>, attr, dev_smem));
-        if constexpr (std::is_same<R, double>::value)
+        if constexpr (std::is_same<R, double>::value) {
+            MLFMA_CK(cudaFuncSetAttribute(t ? k_s2m<R, true> : k_s2m<R, false>, attr, dev_smem));
+            MLFMA_CK(cudaFuncSetAttribute(t ? k_l2t<R, true, true> : k_l2t<R, false, true>, attr, dev_smem));
             MLFMA_CK(cudaFuncSetAttribute(t ? k_m2l_group<true> : k_m2l_group<false>, attr, dev_smem));
+        }
         if constexpr (!std::is_same<R, double>::value) {
             MLFMA_CK(cudaFuncSetAttribute(t ? k_s2m_half<R, true> : k_s2m_half<R, false>, attr, dev_smem));
             MLFMA_CK(cudaFuncSetAttribute(t ? k_l2t_half<R, true> : k_l2t_half<R, false>, attr, dev_smem));
@@ -814,12 +837,12 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
         by_work(s2m_items_h, false);
         by_work(l2t_items, true);
 
-        n_s2m_items_ = static_cast<int>(s2m_items.size());
-        s2m_items_ = upload(s2m_items);
-        n_s2m_items_h_ = static_cast<int>(s2m_items_h.size());
-        if (precision != kFp64) s2m_items_h_ = upload(s2m_items_h);
+        n_s2m_items_[kFp64] = static_cast<int>(s2m_items.size());
+        n_s2m_items_[kMixed] = static_cast<int>(s2m_items_h.size());
         n_l2t_items_ = static_cast<int>(l2t_items.size());
-        l2t_items_ = upload(l2t_items);
+        s2m_items_[kFp64] = std::move(s2m_items);
+        s2m_items_[kMixed] = std::move(s2m_items_h);
+        l2t_items_ = std::move(l2t_items);
         long long far_srcs = 0;
         for (const FarLeaf& f : plan.far_leaves) far_srcs += f.nsrc;
         far_covers_all_ = n_leaves_ > 0 && far_srcs == n_;
@@ -987,14 +1010,12 @@ int DeviceOp::launches_per_matvec() const {
 template <class R, bool TR>
 void DeviceOp::far_s2m(FarField<R>& F, const double2* xt, cudaStream_t s) {
     using C = typename Cx<R>::T;
-    if constexpr (std::is_same<R, double>::value) {
-        if (n_s2m_items_)
-            k_s2m<R, TR><<<n_s2m_items_, kS2MThreads, sizeof(C) * std::max(1, max_src_), s>>>(F.lv_dev, s2m_items_,
-                                                                                                leaves_, F.pat, xt);
-    } else if (n_s2m_items_h_) {
-        k_s2m_half<R, TR><<<n_s2m_items_h_, kS2MThreads, sizeof(C) * std::max(1, max_src_), s>>>(
-            F.lv_dev, s2m_items_h_, leaves_, F.hpat, xt);
-    }
+    constexpr bool f64 = std::is_same<R, double>::value;
+    const int n = n_s2m_items_[f64 ? kFp64 : kMixed];
+    const size_t smem = sizeof(C) * std::max(1, max_src_);
+    if (!n) return;
+    if constexpr (f64) k_s2m<R, TR><<<n, kS2MThreads, smem, s>>>(F.s2m, xt);
+    else k_s2m_half<R, TR><<<n, kS2MThreads, smem, s>>>(F.s2m, xt);
 }
 
 template <class R, bool TR>
@@ -1121,12 +1142,19 @@ void DeviceOp::far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
 
 template <class R, bool TR>
 void DeviceOp::far_l2t(FarField<R>& F, cudaStream_t s, bool pdl) {
-    if (!n_l2t_items_) return;
-    if constexpr (std::is_same<R, double>::value)
-        launch_k(pdl, k_l2t<R, !TR>, n_l2t_items_, kL2TThreads, 0, s, F.lv_dev, l2t_items_, leaves_, F.pat, yfar_);
-    else
-        launch_k(pdl, k_l2t_half<R, !TR>, n_l2t_items_, kL2TThreads, 2 * sizeof(typename Cx<R>::T) * max_leaf_ndir_, s,
-                 F.lv_dev, l2t_items_, leaves_, F.hpat, yfar_);
+    using C = typename Cx<R>::T;
+    constexpr bool f64 = std::is_same<R, double>::value;
+    const int n = n_l2t_items_;
+    const size_t smem = 2 * sizeof(C) * max_leaf_ndir_;  // the local pattern; half patterns: and its antipodal image
+    if (!n) return;
+    if constexpr (f64) {
+        // three blocks to an SM: up to 72 KB each; larger leaf grids (from about
+        // four wavelengths a leaf on) read the local pattern through the L1
+        if (smem <= kL2TStageBytes) launch_k(pdl, k_l2t<R, !TR, true>, n, kL2TThreads, smem, s, F.l2t, yfar_);
+        else launch_k(pdl, k_l2t<R, !TR, false>, n, kL2TThreads, 0, s, F.l2t, yfar_);
+    } else {
+        launch_k(pdl, k_l2t_half<R, !TR>, n, kL2TThreads, smem, s, F.l2t, yfar_);
+    }
 }
 
 // stage: -1 all, 0 S2M, 1 M2M, 2 M2L, 3 L2L, 4 L2T, in sequence on s.
@@ -1174,7 +1202,7 @@ void DeviceOp::run_far_overlap_t(FarField<R>& F, const double2* xt, cudaStream_t
     far_s2m<R, TR>(F, xt, s);
     // chain: the last operation on s is a kernel of the chain (a programmatic
     // dependent launch may follow it), not a memset or a join of side streams
-    bool chain = (std::is_same<R, double>::value ? n_s2m_items_ : n_s2m_items_h_) > 0;
+    bool chain = n_s2m_items_[std::is_same<R, double>::value ? kFp64 : kMixed] > 0;
     cudaEventRecord(ev_level_[lmax_], s);
     if (near_late) {
         cudaStreamWaitEvent(side_, ev_level_[lmax_], 0);

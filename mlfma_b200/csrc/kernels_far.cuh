@@ -38,110 +38,122 @@ __device__ __forceinline__ void chain_wait() {
 // levels in one launch; one thread per element e (direction, component), so
 // every pattern row is read once with coalesced loads; eight sources are in
 // flight per thread.
-constexpr int kS2MThreads = 352;
-constexpr int kL2TThreads = 256;
-constexpr int kL2TSrcPerBlock = kL2TThreads / 32;
+//
+// HBM-bound.  An item carries all its pointers, so a block's first eight rows
+// are requested after one load instead of a chain of three, and while the
+// sources are staged; blocks of 192 threads at 64 registers keep five on an SM
+// (352 at 74 kept two).  One B200: r = 8 sphere 510 -> 420 us (2.75 GB, 6.55 TB/s,
+// the copy rate), complex float 207 -> 130 us (0.69 GB); r = 2 sphere 37 -> 33
+// us, complex float 21 -> 14 us.
+constexpr int kS2MThreads = 192;
+constexpr int kL2TThreads = 128;
+constexpr size_t kL2TStageBytes = 72 * 1024;  // largest local pattern k_l2t stages
+constexpr int kL2TRows = 2;  // sources per warp
+constexpr int kL2TSrcPerBlock = kL2TRows * kL2TThreads / 32;
 
 // CJ: conjugated patterns, a_B[e] = sum_n x_n conj(R_n[e]) -- the transpose of
 // L2T, first stage of the transposed product.
 template <class R, bool CJ>
-__global__ void __launch_bounds__(kS2MThreads)
-k_s2m(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ items, const DevFarLeaf* __restrict__ leaves,
-      const typename Cx<R>::T* __restrict__ pat, const double2* __restrict__ x) {
+__global__ void __launch_bounds__(kS2MThreads, 5)
+k_s2m(const DevS2MItem<R>* __restrict__ items, const double2* __restrict__ x) {
     chain_wait();
     using C = typename Cx<R>::T;
     extern __shared__ unsigned char smraw[];
     C* xs = reinterpret_cast<C*>(smraw);
-    const int4 it = items[blockIdx.x];  // leaf, first element, element count
-    const DevFarLeaf lf = leaves[it.x];
-    const int ne = 2 * lvs[lf.level].ndir;
-    C* A = lvs[lf.level].A + static_cast<size_t>(lf.box) * ne;
-    for (int i = threadIdx.x; i < lf.nsrc; i += blockDim.x) xs[i] = from_d2<C>(x[lf.src0 + i]);
+    const DevS2MItem<R> it = items[blockIdx.x];
+    const int ne = it.ne, nsrc = it.nsrc;
+    const bool live = static_cast<int>(threadIdx.x) < it.ec;
+    const C* r = it.pat + threadIdx.x;
+    C v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        v[u] = live && u < nsrc ? ldg_stream(r + static_cast<size_t>(u) * ne) : zero<C>();
+    for (int i = threadIdx.x; i < nsrc; i += blockDim.x) xs[i] = from_d2<C>(x[it.src0 + i]);
     __syncthreads();
-    if (static_cast<int>(threadIdx.x) >= it.z) return;
-    const int e = it.y + threadIdx.x;
-    const C* r = pat + lf.pat_off * 2 + e;
-    C a0 = zero<C>(), a1 = zero<C>(), a2 = zero<C>(), a3 = zero<C>();
-    int s = 0;
-    for (; s + 8 <= lf.nsrc; s += 8) {
-        C v[8];
+    if (!live) return;
+    C a[4] = {zero<C>(), zero<C>(), zero<C>(), zero<C>()};
+    for (int s = 0;;) {
+        if (s + 8 <= nsrc) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = ldg_stream(r + static_cast<size_t>(s + u) * ne);
-        if (CJ) {
-            a0 = cjfma(v[0], xs[s], a0);
-            a1 = cjfma(v[1], xs[s + 1], a1);
-            a2 = cjfma(v[2], xs[s + 2], a2);
-            a3 = cjfma(v[3], xs[s + 3], a3);
-            a0 = cjfma(v[4], xs[s + 4], a0);
-            a1 = cjfma(v[5], xs[s + 5], a1);
-            a2 = cjfma(v[6], xs[s + 6], a2);
-            a3 = cjfma(v[7], xs[s + 7], a3);
+            for (int u = 0; u < 8; ++u) a[u & 3] = CJ ? cjfma(v[u], xs[s + u], a[u & 3]) : cfma(xs[s + u], v[u], a[u & 3]);
         } else {
-            a0 = cfma(xs[s], v[0], a0);
-            a1 = cfma(xs[s + 1], v[1], a1);
-            a2 = cfma(xs[s + 2], v[2], a2);
-            a3 = cfma(xs[s + 3], v[3], a3);
-            a0 = cfma(xs[s + 4], v[4], a0);
-            a1 = cfma(xs[s + 5], v[5], a1);
-            a2 = cfma(xs[s + 6], v[6], a2);
-            a3 = cfma(xs[s + 7], v[7], a3);
-        }
-    }
-    if (s < lf.nsrc) {  // the last sources: their loads in flight together
-        C v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            v[u] = s + u < lf.nsrc ? ldg_stream(r + static_cast<size_t>(s + u) * ne) : zero<C>();
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (s + u >= lf.nsrc) break;
-            C& acc = (u & 3) == 0 ? a0 : (u & 3) == 1 ? a1 : (u & 3) == 2 ? a2 : a3;
-            acc = CJ ? cjfma(v[u], xs[s + u], acc) : cfma(xs[s + u], v[u], acc);
+            for (int u = 0; u < 8; ++u) {
+                if (s + u >= nsrc) break;
+                a[u & 3] = CJ ? cjfma(v[u], xs[s + u], a[u & 3]) : cfma(xs[s + u], v[u], a[u & 3]);
+            }
         }
+        s += 8;
+        if (s >= nsrc) break;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = s + u < nsrc ? ldg_stream(r + static_cast<size_t>(s + u) * ne) : zero<C>();
     }
-    A[e] = cadd(cadd(a0, a1), cadd(a2, a3));
+    it.a[it.e0 + threadIdx.x] = cadd(cadd(a[0], a[1]), cadd(a[2], a[3]));
 }
 
 // ------------------------------------------------------------ L2T
 // y_m = sum_e conj(R_m[e]) b_B[e]  (Leaf::evalFarSols, src/fmm/leaf.cpp:257-280;
 // C k is applied when the result is written out).  One block per work item
-// (leaf, run of up to eight sources), one warp per source, eight loads in
-// flight per lane; the sum is widened to complex double on output.
+// (leaf, run of up to eight sources), two sources per warp with twelve loads in
+// flight for each and lane, issued before the leaf's local pattern is staged in
+// shared memory; the sum is widened to complex double on output.
+//
+// HBM-bound (latency of the short rows: 3-5 KB a source).  Self-contained items
+// and the early loads: r = 2 sphere 45 -> 39 us, r = 8 sphere 597 -> 575 us
+// (4.8 TB/s); complex float 22 -> 18 us and 246 -> 183 us.  Blocks of 256
+// threads left more warps idle at a leaf's last run of sources (FP64 598 us,
+// complex float 200 us on the r = 8 sphere).
 // CJ = false: plain patterns, y_m = sum_e R_m[e] b_B[e] -- the transpose of S2M,
 // last stage of the transposed product.
-template <class R, bool CJ>
-__global__ void __launch_bounds__(kL2TThreads)
-k_l2t(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ items, const DevFarLeaf* __restrict__ leaves,
-      const typename Cx<R>::T* __restrict__ pat, double2* __restrict__ yfar) {
+template <class R, bool CJ, bool STAGE>  // STAGE: the local pattern in shared memory
+__global__ void __launch_bounds__(kL2TThreads, 4)
+k_l2t(const DevL2TItem<R>* __restrict__ items, double2* __restrict__ yfar) {
     chain_wait();
     using C = typename Cx<R>::T;
-    const int4 it = items[blockIdx.x];  // leaf, first source, source count
+    constexpr int RW = kL2TRows, U = 12;
+    extern __shared__ unsigned char smraw[];
+    C* bs = reinterpret_cast<C*>(smraw);
+    const DevL2TItem<R> it = items[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp >= it.z) return;
-    const DevFarLeaf lf = leaves[it.x];
-    const int ndir = lvs[lf.level].ndir, ne = 2 * ndir;
-    const C* Bb = lvs[lf.level].B + static_cast<size_t>(lf.box) * ne;
-    const int s = it.y + warp;
-    const C* r = pat + (lf.pat_off + static_cast<long long>(s) * ndir) * 2;
-    C a0 = zero<C>(), a1 = zero<C>(), a2 = zero<C>(), a3 = zero<C>();
-    // eight loads in flight per lane, the last run of the row predicated (a
-    // leaf-level row of 162-324 elements is one or two runs)
-    for (int e = lane; e < ne; e += 256) {
-        C v[8], bv[8];
+    const int ne = it.ne;
+    C v[RW][U];  // the rows' first runs, in flight while the local pattern is staged
+    auto load = [&](int e) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const bool in = e + 32 * u < ne;
-            v[u] = in ? ldg_stream(r + e + 32 * u) : zero<C>();
-            bv[u] = in ? Bb[e + 32 * u] : zero<C>();
-        }
+        for (int q = 0; q < RW; ++q) {
+            const int row = warp + q * (kL2TThreads / 32);
+            const C* r = it.pat + static_cast<size_t>(row) * ne;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            C& acc = (u & 3) == 0 ? a0 : (u & 3) == 1 ? a1 : (u & 3) == 2 ? a2 : a3;
-            acc = CJ ? cjfma(v[u], bv[u], acc) : cfma(v[u], bv[u], acc);
+            for (int u = 0; u < U; ++u)
+                v[q][u] = row < it.cnt && e + 32 * u < ne ? ldg_stream(r + e + 32 * u) : zero<C>();
         }
+    };
+    load(lane);
+    if (STAGE) {
+        for (int e = threadIdx.x; e < ne; e += blockDim.x) bs[e] = it.b[e];
+        __syncthreads();
     }
-    const C acc = warp_sum(cadd(cadd(a0, a1), cadd(a2, a3)));
-    if (lane == 0) yfar[lf.src0 + s] = to_d2(acc);
+    const C* b = STAGE ? bs : it.b;
+    C a[RW][2];
+#pragma unroll
+    for (int q = 0; q < RW; ++q) a[q][0] = a[q][1] = zero<C>();
+    for (int e = lane;;) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (e + 32 * u >= ne) continue;
+            const C bv = b[e + 32 * u];
+#pragma unroll
+            for (int q = 0; q < RW; ++q) a[q][u & 1] = CJ ? cjfma(v[q][u], bv, a[q][u & 1]) : cfma(v[q][u], bv, a[q][u & 1]);
+        }
+        e += 32 * U;
+        if (e - lane >= ne) break;  // (the whole warp: the sums below shuffle)
+        load(e);
+    }
+#pragma unroll
+    for (int q = 0; q < RW; ++q) {
+        const C acc = warp_sum(cadd(a[q][0], a[q][1]));
+        const int row = warp + q * (kL2TThreads / 32);
+        if (lane == 0 && row < it.cnt) yfar[it.src0 + row] = to_d2(acc);
+    }
 }
 
 // Half patterns (the complex-float far field of the mixed operator): patterns
@@ -178,132 +190,115 @@ __global__ void k_half_patterns(const DevLevelT<R>* __restrict__ lvs, const DevF
 // first half), all leaf levels in one launch; one thread per element e, which
 // also forms the antipodal element a_B[anti[e]] = sgn sum_n x_n conj(R_n[e]);
 // every stored pattern row is read once with coalesced loads; eight sources
-// are in flight per thread.
+// are in flight per thread, the first before the sources are staged (as k_s2m).
 // CJ: conjugated patterns, a_B[e] = sum_n x_n conj(R_n[e]) -- the transpose of
 // L2T, first stage of the transposed product.
 template <class R, bool CJ>
 __global__ void __launch_bounds__(kS2MThreads)
-k_s2m_half(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ items, const DevFarLeaf* __restrict__ leaves,
-      const typename Cx<R>::T* __restrict__ hpat, const double2* __restrict__ x) {
+k_s2m_half(const DevS2MItem<R>* __restrict__ items, const double2* __restrict__ x) {
     chain_wait();
     using C = typename Cx<R>::T;
     extern __shared__ unsigned char smraw[];
     C* xs = reinterpret_cast<C*>(smraw);
-    const int4 it = items[blockIdx.x];  // leaf, first element, element count
-    const DevFarLeaf lf = leaves[it.x];
-    const DevLevelT<R> lv = lvs[lf.level];
-    const int ne = lv.ndir;  // stored elements per source
-    C* A = lv.A + static_cast<size_t>(lf.box) * 2 * ne;
-    for (int i = threadIdx.x; i < lf.nsrc; i += blockDim.x) xs[i] = from_d2<C>(x[lf.src0 + i]);
+    const DevS2MItem<R> it = items[blockIdx.x];
+    const int ne = it.ne, nsrc = it.nsrc;  // ne: stored elements per source
+    const bool live = static_cast<int>(threadIdx.x) < it.ec;
+    const C* r = it.pat + threadIdx.x;
+    C v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        v[u] = live && u < nsrc ? ldg_stream(r + static_cast<size_t>(u) * ne) : zero<C>();
+    const int e = it.e0 + threadIdx.x;
+    const int ea = live ? it.anti[e] : 0;
+    for (int i = threadIdx.x; i < nsrc; i += blockDim.x) xs[i] = from_d2<C>(x[it.src0 + i]);
     __syncthreads();
-    if (static_cast<int>(threadIdx.x) >= it.z) return;
-    const int e = it.y + threadIdx.x;
-    const C* r = hpat + lf.pat_off + e;
+    if (!live) return;
     // a: this element, b: sum of x conj(v) (or x v), the antipodal one up to its sign
-    C a0 = zero<C>(), a1 = zero<C>(), a2 = zero<C>(), a3 = zero<C>();
-    C b0 = zero<C>(), b1 = zero<C>(), b2 = zero<C>(), b3 = zero<C>();
-    int s = 0;
-    for (; s + 8 <= lf.nsrc; s += 8) {
-        C v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = ldg_stream(r + static_cast<size_t>(s + u) * ne);
-#pragma unroll
-        for (int u = 0; u < 8; u += 4) {
-            if (CJ) {
-                a0 = cjfma(v[u], xs[s + u], a0);
-                a1 = cjfma(v[u + 1], xs[s + u + 1], a1);
-                a2 = cjfma(v[u + 2], xs[s + u + 2], a2);
-                a3 = cjfma(v[u + 3], xs[s + u + 3], a3);
-                b0 = cfma(xs[s + u], v[u], b0);
-                b1 = cfma(xs[s + u + 1], v[u + 1], b1);
-                b2 = cfma(xs[s + u + 2], v[u + 2], b2);
-                b3 = cfma(xs[s + u + 3], v[u + 3], b3);
-            } else {
-                a0 = cfma(xs[s + u], v[u], a0);
-                a1 = cfma(xs[s + u + 1], v[u + 1], a1);
-                a2 = cfma(xs[s + u + 2], v[u + 2], a2);
-                a3 = cfma(xs[s + u + 3], v[u + 3], a3);
-                b0 = cjfma(v[u], xs[s + u], b0);
-                b1 = cjfma(v[u + 1], xs[s + u + 1], b1);
-                b2 = cjfma(v[u + 2], xs[s + u + 2], b2);
-                b3 = cjfma(v[u + 3], xs[s + u + 3], b3);
-            }
-        }
-    }
-    if (s < lf.nsrc) {  // the last sources: their loads in flight together
-        C v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            v[u] = s + u < lf.nsrc ? ldg_stream(r + static_cast<size_t>(s + u) * ne) : zero<C>();
+    C a[4] = {zero<C>(), zero<C>(), zero<C>(), zero<C>()};
+    C b[4] = {zero<C>(), zero<C>(), zero<C>(), zero<C>()};
+    for (int s = 0;;) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (s + u >= lf.nsrc) break;
-            C& a = (u & 3) == 0 ? a0 : (u & 3) == 1 ? a1 : (u & 3) == 2 ? a2 : a3;
-            C& b = (u & 3) == 0 ? b0 : (u & 3) == 1 ? b1 : (u & 3) == 2 ? b2 : b3;
-            a = CJ ? cjfma(v[u], xs[s + u], a) : cfma(xs[s + u], v[u], a);
-            b = CJ ? cfma(xs[s + u], v[u], b) : cjfma(v[u], xs[s + u], b);
+            if (s + u >= nsrc) break;
+            const C xv = xs[s + u];
+            a[u & 3] = CJ ? cjfma(v[u], xv, a[u & 3]) : cfma(xv, v[u], a[u & 3]);
+            b[u & 3] = CJ ? cfma(xv, v[u], b[u & 3]) : cjfma(v[u], xv, b[u & 3]);
         }
+        s += 8;
+        if (s >= nsrc) break;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = s + u < nsrc ? ldg_stream(r + static_cast<size_t>(s + u) * ne) : zero<C>();
     }
-    A[e] = cadd(cadd(a0, a1), cadd(a2, a3));
-    const C b = cadd(cadd(b0, b1), cadd(b2, b3));
-    A[lv.anti[e]] = (e & 1) ? C{-b.x, -b.y} : b;
+    it.a[e] = cadd(cadd(a[0], a[1]), cadd(a[2], a[3]));
+    const C q = cadd(cadd(b[0], b[1]), cadd(b[2], b[3]));
+    it.a[ea] = (e & 1) ? C{-q.x, -q.y} : q;
 }
 
 // ------------------------------------------------------------ L2T, half patterns
 // y_m = sum_e conj(R_m[e]) b_B[e] over the stored half:
 // y_m = sum_{e < ndir} conj(R_m[e]) b_B[e] + R_m[e] b'_B[e], b'_B[e] =
 // sgn(e) b_B[anti[e]].  One block per work item (leaf, run of up to eight
-// sources): the block first stages b_B and b'_B in shared memory, then one warp
-// per source streams its stored patterns (eight loads in flight per lane).
+// sources): two sources per warp, eight loads in flight for each and lane,
+// issued before the block stages b_B and b'_B in shared memory (as k_l2t).
 // CJ = false: plain patterns (the transpose of S2M).
 template <class R, bool CJ>
 __global__ void __launch_bounds__(kL2TThreads)
-k_l2t_half(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ items, const DevFarLeaf* __restrict__ leaves,
-           const typename Cx<R>::T* __restrict__ hpat, double2* __restrict__ yfar) {
+k_l2t_half(const DevL2TItem<R>* __restrict__ items, double2* __restrict__ yfar) {
     chain_wait();
     using C = typename Cx<R>::T;
+    constexpr int RW = kL2TRows, U = 8;
     extern __shared__ unsigned char smraw[];
-    const int4 it = items[blockIdx.x];  // leaf, first source, source count
+    const DevL2TItem<R> it = items[blockIdx.x];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const DevFarLeaf lf = leaves[it.x];
-    const DevLevelT<R> lv = lvs[lf.level];
-    const int ne = lv.ndir;  // stored elements per source
+    const int ne = it.ne;  // stored elements per source
+    C v[RW][U];  // the rows' first runs, in flight while the local pattern is staged
+    auto load = [&](int e) {
+#pragma unroll
+        for (int q = 0; q < RW; ++q) {
+            const int row = warp + q * (kL2TThreads / 32);
+            const C* r = it.pat + static_cast<size_t>(row) * ne;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[q][u] = row < it.cnt && e + 32 * u < ne ? ldg_stream(r + e + 32 * u) : zero<C>();
+        }
+    };
+    load(lane);
     C* bs = reinterpret_cast<C*>(smraw);
     C* bp = bs + ne;
-    {
-        const C* Bb = lv.B + static_cast<size_t>(lf.box) * 2 * ne;
-        for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-            bs[e] = Bb[e];
-            const C q = Bb[lv.anti[e]];
-            bp[e] = (e & 1) ? C{-q.x, -q.y} : q;
-        }
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+        const C q = it.b[it.anti[e]];
+        bs[e] = it.b[e];
+        bp[e] = (e & 1) ? C{-q.x, -q.y} : q;
     }
     __syncthreads();
-    if (warp >= it.z) return;
-    const int s = it.y + warp;
-    const C* r = hpat + lf.pat_off + static_cast<long long>(s) * ne;
-    C a0 = zero<C>(), a1 = zero<C>(), a2 = zero<C>(), a3 = zero<C>();
-    // eight loads in flight per lane, the last run of the row predicated
-    for (int e = lane; e < ne; e += 256) {
-        C v[8];
+    C a[RW][4];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = e + 32 * u < ne ? ldg_stream(r + e + 32 * u) : zero<C>();
+    for (int q = 0; q < RW; ++q)
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int k = 0; k < 4; ++k) a[q][k] = zero<C>();
+    for (int e = lane;;) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
             const int ee = e + 32 * u;
             if (ee >= ne) continue;
-            C& acc = (u & 3) == 0 ? a0 : (u & 3) == 1 ? a1 : (u & 3) == 2 ? a2 : a3;
-            if (CJ) {
-                acc = cjfma(v[u], bs[ee], acc);
-                acc = cfma(v[u], bp[ee], acc);
-            } else {
-                acc = cfma(v[u], bs[ee], acc);
-                acc = cjfma(v[u], bp[ee], acc);
+            const C b0 = bs[ee], b1 = bp[ee];
+#pragma unroll
+            for (int q = 0; q < RW; ++q) {
+                C& acc = a[q][u & 3];
+                acc = CJ ? cjfma(v[q][u], b0, acc) : cfma(v[q][u], b0, acc);
+                acc = CJ ? cfma(v[q][u], b1, acc) : cjfma(v[q][u], b1, acc);
             }
         }
+        e += 32 * U;
+        if (e - lane >= ne) break;  // (the whole warp: the sums below shuffle)
+        load(e);
     }
-    const C acc = warp_sum(cadd(cadd(a0, a1), cadd(a2, a3)));
-    if (lane == 0) yfar[lf.src0 + s] = to_d2(acc);
+#pragma unroll
+    for (int q = 0; q < RW; ++q) {
+        const C acc = warp_sum(cadd(cadd(a[q][0], a[q][1]), cadd(a[q][2], a[q][3])));
+        const int row = warp + q * (kL2TThreads / 32);
+        if (lane == 0 && row < it.cnt) yfar[it.src0 + row] = to_d2(acc);
+    }
 }
 
 // ------------------------------------------------------------ M2M
