@@ -194,7 +194,7 @@ struct TuneReport {
                                    // S2M, bit 2 two side streams for the finer levels' M2L, bit 3
                                    // chain kernels as programmatic dependent launches
     int m2m_staged, l2l_staged;    // one-vector: bit p = transition p -> p + 1 on the staged kernels
-    int near_kernel;               // one-vector near field: 0 k_near_sym, 1 k_near_warp
+    int near_kernel;               // one-vector near field: 0 k_near_sym, 2 k_near_direct
 };
 
 // Tensor-core interpolation and anterpolation of one level transition
@@ -295,7 +295,7 @@ public:
     // bit 0: every transition's M2M on k_m2m_sum, bit 1: L2L on k_l2l_st (where they fit)
     std::string set_staged(int mode);
     std::string set_schedule(int schedule);
-    std::string set_near_kernel(int kind);  // 0 k_near_sym, 1 k_near_warp
+    std::string set_near_kernel(int kind);  // 0 k_near_sym, 1 or 2 k_near_direct
     // per level l (index l): M2M into l, M2L at l, L2L out of l (ms; 0 where none)
     std::string time_levels(std::vector<float>& out);
     // Chooses launch shapes by timing them on this operator (see kernels.cu).
@@ -356,8 +356,8 @@ private:
     template <class R> std::string setup_far(const Plan& plan, FarField<R>& F, const double2* pat64);
     template <class R, bool TR> void run_far_t(FarField<R>& F, const double2* xt, cudaStream_t s, int stage);
     template <class R, bool TR> void run_far_overlap_t(FarField<R>& F, const double2* xt, cudaStream_t s,
-                                                       cudaStream_t s2, bool near_late);
-    void run_far_overlap(const double2* xt, cudaStream_t s, cudaStream_t s2, int prec, bool tr, bool late);
+                                                       cudaStream_t s2, bool near_late, bool krylov);
+    void run_far_overlap(const double2* xt, cudaStream_t s, cudaStream_t s2, int prec, bool tr, bool late, bool krylov);
     // pdl: launched as a programmatic dependent launch (the predecessor on s
     // is a kernel of the chain, and the only one this launch depends on)
     template <class R, bool TR> void far_s2m(FarField<R>& F, const double2* xt, cudaStream_t s);
@@ -366,9 +366,10 @@ private:
     template <class R, bool TR> void far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl = false);
     template <class R, bool TR> void far_l2t(FarField<R>& F, cudaStream_t s, bool pdl = false);
     void run_far(const double2* xt, cudaStream_t s, int stage = -1, int prec = -1, bool tr = false);
-    void run_near(const double2* xt, cudaStream_t s);
-    void enqueue_core(cudaStream_t s, int prec, bool tr);   // xt_ -> yfar_, ynear_
-    void launch_core(cudaStream_t s, int prec, bool tr);
+    void run_near(const double2* xt, cudaStream_t s, bool krylov = false);
+    // xt_ -> yfar_, ynear_; krylov: a product of a solve (see run_near)
+    void enqueue_core(cudaStream_t s, int prec, bool tr, bool krylov = false);
+    void launch_core(cudaStream_t s, int prec, bool tr, bool krylov);
     template <class R> void run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage);
     void run_far_multi(int nr, cudaStream_t s, int stage, int prec);
     void run_near_multi(int nr, cudaStream_t s);
@@ -378,7 +379,7 @@ private:
     size_t m2l_item_capacity(int min_chunk) const;
     void build_m2l_items(int max_chunk);
     std::string build_m2l_families(const Plan& plan);
-    std::string ensure_graph(int prec, bool tr);
+    std::string ensure_graph(int prec, bool tr, bool krylov);
     std::string setup_tc(const Plan& plan);
     std::string build_transl_device(const Level& L, double2* t);
     void far_m2m_tc(int p, int nr, cudaStream_t s);
@@ -395,8 +396,8 @@ private:
     cudaEvent_t ev_level_[kMaxLevels] = {};  // outgoing patterns of a level final
     std::vector<void*> allocs_;
     long long bytes_ = 0;
-    cudaGraph_t graph_[2][2] = {};          // per far-field precision, forward / transposed
-    cudaGraphExec_t graph_exec_[2][2] = {};
+    cudaGraph_t graph_[2][2][2] = {};       // per far-field precision, forward / transposed, solve (mixed operators)
+    cudaGraphExec_t graph_exec_[2][2][2] = {};
     bool use_graph_ = true;
 
     // Shared by both precisions.
@@ -417,13 +418,20 @@ private:
     int m2l_chunk_ = 128;                 // one-vector M2L directions per block
     int m2l_staged_ = 1;                  // one-vector M2L with its lists staged in shared memory
     bool near_late_ = false;              // near field after S2M (overlapping the latency-bound stages)
-    int m2l_streams_ = 1;                 // side streams for the finer levels' translations
+    // side streams for the finer levels' translations: two (r = 2 sphere FP64 189
+    // -> 184 us, r = 4 sphere 751 -> 737 us, 50,000 dipoles 604 -> 599 us)
+    int m2l_streams_ = 2;
     bool chain_pdl_ = false;              // far-field chain kernels as programmatic dependent launches
     std::vector<int> m2m_rows_;           // one-vector M2M parent rows per block, per transition
     std::vector<int> m2m_pref_, l2l_pref_;  // per transition: 1 = staged kernels (k_m2m_sum, k_l2l_st) where they fit
     int dev_smem_ = 0;                    // opt-in shared memory per block
-    int near_kernel_ = 0;                 // one-vector near field: 0 k_near_sym, 1 k_near_warp, 2 k_near_direct
+    int near_kernel_ = 0;                 // one-vector near field: 0 k_near_sym, 1 or 2 k_near_direct (where there are quads)
     int near_direct_occ_ = 1;             // k_near_direct blocks per SM
+    DevNearTile* near_quads_ = nullptr;   // k_near_direct: tiles in groups of four of like shape,
+    int n_near_quads_ = 0;
+    int* near_qslot_ = nullptr;           //   slots of their partials
+    int* near_qred_ptr_ = nullptr;        //   and [n + 1]: target t's slots
+    int near_sym_grid_ = 0;               // k_near_sym in products of a mixed operator's solves
     int m_m2m_rows_fast_ = -1;            // many-rhs M2M grid order (-1: precision default)
     int m_l2l_pairs_ = 0;                 // many-rhs L2L column pairs per block (0: precision default)
     std::vector<int2*> l2l_pairs_;       // per parent level: (parent, child entry)

@@ -142,11 +142,7 @@ constexpr int kDnWidths[] = {8, 12, 16, 24, 32};
 
 DeviceOp::~DeviceOp() {
     if (device_ >= 0) cudaSetDevice(device_);
-    for (int p = 0; p < 2; ++p)
-        for (int t = 0; t < 2; ++t) {
-            if (graph_exec_[p][t]) cudaGraphExecDestroy(graph_exec_[p][t]);
-            if (graph_[p][t]) cudaGraphDestroy(graph_[p][t]);
-        }
+    drop_graphs();
     for (void* p : allocs_) cudaFree(p);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     if (ev_join_) cudaEventDestroy(ev_join_);
@@ -165,9 +161,8 @@ DeviceOp::~DeviceOp() {
 // block, so that a small operator leaves room for the kernels of others
 // running beside it.
 void DeviceOp::set_near_grid(int per_sm) {
-    if (near_kernel_ == 1) per_sm = 1;  // k_near_warp: one block per SM (its ring fills the shared memory)
-    if (near_kernel_ == 2) {            // k_near_direct: every resident warp of the grid takes tiles
-        near_grid_ = std::max(1, std::min((n_near_tiles_ + kNdThreads / 32 - 1) / (kNdThreads / 32),
+    if (near_kernel_ != 0 && n_near_quads_) {  // k_near_direct: every resident warp of the grid takes quads
+        near_grid_ = std::max(1, std::min((n_near_quads_ + kNdThreads / 32 - 1) / (kNdThreads / 32),
                                           std::max(1, per_sm) * sms_));
         return;
     }
@@ -745,7 +740,9 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
         build_m2l_items(128);
         MLFMA_CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
         {
-            const std::string e = build_m2l_families(plan);
+            // (a mixed operator's FP64 far field serves its solves' residuals:
+            // it keeps the order of its sums, see run_near)
+            const std::string e = precision == kFp64 ? build_m2l_families(plan) : std::string();
             if (!e.empty()) return e;
         }
 
@@ -914,20 +911,48 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
             n_near_tiles_ = static_cast<int>(nt.size());
             if (n_near_tiles_ > 0) {
                 near_tiles_ = upload(nt);
-                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_));
-                near_part_ = alloc<double2>(static_cast<size_t>(plan.near_parts));
+                size_t parts = plan.near_parts;
+                if (!plan.near_quads.tiles.empty()) {
+                    parts = std::max<size_t>(parts, plan.near_quads.parts);
+                    near_qslot_ = upload(plan.near_quads.slot);
+                    near_qred_ptr_ = upload(plan.near_quads.red_ptr);
+                    // four tiles of like shape per warp: rectangular tiles, then
+                    // self tiles, each by column groups and rows, padded with empty ones
+                    std::vector<DevNearTile> quads;
+                    for (int self = 0; self < 2; ++self) {
+                        const size_t first = quads.size();
+                        for (const NearTile& t : plan.near_quads.tiles)
+                            if ((t.kind != 0) == (self != 0))
+                                quads.push_back(DevNearTile{t.z, t.r0, t.c0, t.i0, t.ni, t.j0, t.nj, t.ld, t.kind,
+                                                            t.slot, t.mode});
+                        std::stable_sort(quads.begin() + first, quads.end(), [](const DevNearTile& a, const DevNearTile& b) {
+                            const int ga = (a.nj + 7) / 8, gb = (b.nj + 7) / 8;
+                            return ga != gb ? ga > gb : a.ni > b.ni;
+                        });
+                        while (quads.size() % 4) {
+                            DevNearTile t{};
+                            t.kind = quads.back().kind;
+                            quads.push_back(t);
+                        }
+                    }
+                    n_near_quads_ = static_cast<int>(quads.size() / 4);
+                    near_quads_ = upload(quads);
+                }
+                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_) + kNearPad);
+                MLFMA_CK(cudaMemsetAsync(near_bz_ + near_block_entries_, 0, sizeof(double2) * kNearPad, stream_));
+                near_part_ = alloc<double2>(parts);
                 near_red_ptr_ = upload(plan.near_red_ptr);
                 near_slot_ = upload(plan.near_slot);
                 MLFMA_CK(cudaFuncSetAttribute(k_near_sym, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(kSymSmemBytes)));
-                MLFMA_CK(cudaFuncSetAttribute(k_near_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(kNwSmemBytes)));
                 MLFMA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&near_occ_, k_near_sym, kSymThreads,
                                                                        kSymSmemBytes));
                 near_occ_ = std::max(1, near_occ_);
                 MLFMA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&near_direct_occ_, k_near_direct, kNdThreads, 0));
                 near_direct_occ_ = std::max(1, near_direct_occ_);
-                near_per_sm_ = near_occ_;
+                near_kernel_ = n_near_quads_ ? 2 : 0;
+                near_sym_grid_ = std::max(1, std::min(n_near_tiles_ / 4, near_occ_ * sms_));
+                near_per_sm_ = near_kernel_ ? near_direct_occ_ : near_occ_;
                 set_near_grid(near_per_sm_);
                 DevNearBlock* d_nb = upload(nb);
                 k_near_blocks_assemble<<<blocks_for(near_block_entries_, 128), 128, 0, stream_>>>(
@@ -1191,7 +1216,7 @@ void DeviceOp::run_far_t(FarField<R>& F, const double2* xt, cudaStream_t s, int 
 // side streams (s2, side3_).
 template <class R, bool TR>
 void DeviceOp::run_far_overlap_t(FarField<R>& F, const double2* xt, cudaStream_t s, cudaStream_t s2,
-                                 bool near_late) {
+                                 bool near_late, bool krylov) {
     if (n_leaves_ == 0) return;
     if (lmax_ <= lmin_) {  // one far level: nothing to overlap
         run_far_t<R, TR>(F, xt, s, -1);
@@ -1206,7 +1231,7 @@ void DeviceOp::run_far_overlap_t(FarField<R>& F, const double2* xt, cudaStream_t
     cudaEventRecord(ev_level_[lmax_], s);
     if (near_late) {
         cudaStreamWaitEvent(side_, ev_level_[lmax_], 0);
-        run_near(xt_, side_);
+        run_near(xt_, side_, krylov);
         cudaEventRecord(ev_join_, side_);
     }
     for (int p = lmax_ - 1; p >= lmin_; --p) {
@@ -1245,33 +1270,37 @@ void DeviceOp::run_far(const double2* xt, cudaStream_t s, int stage, int prec, b
     }
 }
 
-void DeviceOp::run_far_overlap(const double2* xt, cudaStream_t s, cudaStream_t s2, int prec, bool tr, bool late) {
+void DeviceOp::run_far_overlap(const double2* xt, cudaStream_t s, cudaStream_t s2, int prec, bool tr, bool late,
+                               bool krylov) {
     if (prec < 0) prec = precision_;
     if (prec == kFp64) {
-        if (tr) run_far_overlap_t<double, true>(f64_, xt, s, s2, late);
-        else run_far_overlap_t<double, false>(f64_, xt, s, s2, late);
+        if (tr) run_far_overlap_t<double, true>(f64_, xt, s, s2, late, krylov);
+        else run_far_overlap_t<double, false>(f64_, xt, s, s2, late, krylov);
     } else {
-        if (tr) run_far_overlap_t<float, true>(f32_, xt, s, s2, late);
-        else run_far_overlap_t<float, false>(f32_, xt, s, s2, late);
+        if (tr) run_far_overlap_t<float, true>(f32_, xt, s, s2, late, krylov);
+        else run_far_overlap_t<float, false>(f32_, xt, s, s2, late, krylov);
     }
 }
 
-void DeviceOp::run_near(const double2* xt, cudaStream_t s) {
+// krylov: a product of a solve.  On a mixed operator those keep k_near_sym and
+// its order of sums: an inner solve on the complex-float far field rounds its
+// vectors to float, so a change in the last FP64 bit of a product turns some of
+// them and grows to 1e-8 of the solution in fifty iterations (r = 1.83 sphere).
+void DeviceOp::run_near(const double2* xt, cudaStream_t s, bool krylov) {
     if (n_near_tiles_ == 0) {
         cudaMemsetAsync(ynear_, 0, sizeof(double2) * n_, s);
         return;
     }
-    if (near_kernel_ == 2)
-        k_near_direct<<<near_grid_, kNdThreads, 0, s>>>(near_tiles_, n_near_tiles_, near_bz_, xt, near_slot_,
+    const bool ordered = krylov && precision_ != kFp64;
+    const bool quads = near_kernel_ && n_near_quads_ && !ordered;
+    if (quads)
+        k_near_direct<<<near_grid_, kNdThreads, 0, s>>>(near_quads_, n_near_quads_, near_bz_, xt, near_qslot_,
                                                          near_part_);
-    else if (near_kernel_ == 1)
-        k_near_warp<<<near_grid_, kNwThreads, kNwSmemBytes, s>>>(near_tiles_, n_near_tiles_, near_bz_, xt, near_slot_,
-                                                                 near_part_, err_dev_);
     else
-        k_near_sym<<<near_grid_, kSymThreads, kSymSmemBytes, s>>>(near_tiles_, n_near_tiles_, near_bz_, xt, near_slot_,
-                                                                 near_part_, err_dev_);
-    k_near_reduce<<<blocks_for(static_cast<long long>(n_) * kReduceLanes, 256), 256, 0, s>>>(near_red_ptr_, near_part_,
-                                                                                           n_, ynear_);
+        k_near_sym<<<ordered ? near_sym_grid_ : near_grid_, kSymThreads, kSymSmemBytes, s>>>(
+            near_tiles_, n_near_tiles_, near_bz_, xt, near_slot_, near_part_, err_dev_);
+    k_near_reduce<<<blocks_for(static_cast<long long>(n_) * kReduceLanes, 256), 256, 0, s>>>(
+        quads ? near_qred_ptr_ : near_red_ptr_, near_part_, n_, ynear_);
 }
 
 // The tree-ordered product xt_ -> (yfar_, ynear_): near field on the side
@@ -1279,7 +1308,7 @@ void DeviceOp::run_near(const double2* xt, cudaStream_t s) {
 // Captured once per (precision, direction) into a CUDA graph.  The near field
 // is symmetric (each stored block is applied as Z and Z^T), so the transposed
 // product reuses it; run_near writes every entry of ynear_.
-void DeviceOp::enqueue_core(cudaStream_t s, int prec, bool tr) {
+void DeviceOp::enqueue_core(cudaStream_t s, int prec, bool tr, bool krylov) {
     // L2T writes (not adds) every far-leaf source's entry: zero yfar_ only
     // when some source sits in a leaf without far interactions
     if (!far_covers_all_) cudaMemsetAsync(yfar_, 0, sizeof(double2) * n_, s);
@@ -1287,26 +1316,26 @@ void DeviceOp::enqueue_core(cudaStream_t s, int prec, bool tr) {
     const bool late = near_late_ && n_leaves_ > 0 && lmax_ > lmin_;
     if (!late) {
         cudaStreamWaitEvent(side_, ev_fork_, 0);
-        run_near(xt_, side_);
+        run_near(xt_, side_, krylov);
         cudaEventRecord(ev_join_, side_);
     }
-    run_far_overlap(xt_, s, side2_, prec, tr, late);
+    run_far_overlap(xt_, s, side2_, prec, tr, late, krylov);
     cudaStreamWaitEvent(s, ev_join_, 0);
 }
 
-std::string DeviceOp::ensure_graph(int prec, bool tr) {
-    const int t = tr ? 1 : 0;
-    if (graph_exec_[prec][t] || !use_graph_) return {};
+std::string DeviceOp::ensure_graph(int prec, bool tr, bool krylov) {
+    const int t = tr ? 1 : 0, k = krylov && precision_ != kFp64 ? 1 : 0;
+    if (graph_exec_[prec][t][k] || !use_graph_) return {};
     MLFMA_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    enqueue_core(stream_, prec, tr);
-    MLFMA_CK(cudaStreamEndCapture(stream_, &graph_[prec][t]));
-    MLFMA_CK(cudaGraphInstantiate(&graph_exec_[prec][t], graph_[prec][t], cudaGraphInstantiateFlagUseNodePriority));
+    enqueue_core(stream_, prec, tr, krylov);
+    MLFMA_CK(cudaStreamEndCapture(stream_, &graph_[prec][t][k]));
+    MLFMA_CK(cudaGraphInstantiate(&graph_exec_[prec][t][k], graph_[prec][t][k], cudaGraphInstantiateFlagUseNodePriority));
     return {};
 }
 
-void DeviceOp::launch_core(cudaStream_t s, int prec, bool tr) {
-    const int t = tr ? 1 : 0;
-    if (graph_exec_[prec][t]) cudaGraphLaunch(graph_exec_[prec][t], s); else enqueue_core(s, prec, tr);
+void DeviceOp::launch_core(cudaStream_t s, int prec, bool tr, bool krylov) {
+    const int t = tr ? 1 : 0, k = krylov && precision_ != kFp64 ? 1 : 0;
+    if (graph_exec_[prec][t][k]) cudaGraphLaunch(graph_exec_[prec][t][k], s); else enqueue_core(s, prec, tr, krylov);
 }
 
 std::string DeviceOp::set_loads(const double2* z_user) {
@@ -1329,17 +1358,17 @@ std::string DeviceOp::set_loads(const double2* z_user) {
 // Tree-ordered y = A x (adj: y = A^H x = conj(A^T conj(x))), loads included.
 void DeviceOp::apply_tree(const double2* xt, double2* yt, cudaStream_t s, int prec, bool adj) {
     if (prec < 0) prec = precision_;
-    if (!ensure_graph(prec, adj).empty()) use_graph_ = false;
+    if (!ensure_graph(prec, adj, true).empty()) use_graph_ = false;
     if (adj) k_conj_copy<<<blocks_for(n_, 256), 256, 0, s>>>(xt, xt_, n_);
     else if (xt != xt_) cudaMemcpyAsync(xt_, xt, sizeof(double2) * n_, cudaMemcpyDeviceToDevice, s);
-    launch_core(s, prec, adj);
+    launch_core(s, prec, adj, true);
     k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, nullptr, yt, n_, ck_, 0, xt_,
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
 }
 
 void DeviceOp::enqueue_apply_from_input(double2* yt, cudaStream_t s, int prec, bool adj) {
     if (prec < 0) prec = precision_;
-    enqueue_core(s, prec, adj);
+    enqueue_core(s, prec, adj, true);
     k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, nullptr, yt, n_, ck_, 0, xt_,
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
 }
@@ -1348,7 +1377,7 @@ void DeviceOp::apply_tree_direct(const double2* xt, double2* yt, cudaStream_t s,
     if (prec < 0) prec = precision_;
     if (adj) k_conj_copy<<<blocks_for(n_, 256), 256, 0, s>>>(xt, xt_, n_);
     else if (xt != xt_) cudaMemcpyAsync(xt_, xt, sizeof(double2) * n_, cudaMemcpyDeviceToDevice, s);
-    launch_core(s, prec, adj);
+    launch_core(s, prec, adj, true);
     k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, nullptr, yt, n_, ck_, 0, xt_,
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
 }
@@ -1361,10 +1390,10 @@ std::string DeviceOp::matvec_device(const double2* x, double2* y, bool accumulat
     if (adj && ref_compat_) return "arg:the adjoint needs ref_compat = 0 (the reference's rule keeps state between products)";
     cudaStream_t s = stream ? stream : stream_;
     MLFMA_CK(cudaSetDevice(device_));
-    std::string e = ensure_graph(prec, adj);
+    std::string e = ensure_graph(prec, adj, false);
     if (!e.empty()) return e;
     k_gather<<<blocks_for(n_, 256), 256, 0, s>>>(x, perm_, xt_, n_, adj ? 1 : 0);
-    launch_core(s, prec, adj);
+    launch_core(s, prec, adj, false);
     k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, perm_, y, n_, ck_, accumulate ? 1 : 0, xt_,
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
     MLFMA_CK(cudaGetLastError());
@@ -1375,10 +1404,10 @@ std::string DeviceOp::matvec_mapped(const double2* x, double2* y, bool accumulat
     if (!ready_) return "operator not set up";
     cudaStream_t s = stream ? stream : stream_;
     MLFMA_CK(cudaSetDevice(device_));
-    std::string e = ensure_graph(precision_, false);
+    std::string e = ensure_graph(precision_, false, false);
     if (!e.empty()) return e;
     k_gather_caller<<<blocks_for(n_, 256), 256, 0, s>>>(x, tpos_, xt_, n_);
-    launch_core(s, precision_, false);
+    launch_core(s, precision_, false, false);
     k_finish_caller<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, tpos_, y, n_, ck_, accumulate ? 1 : 0, xt_,
                                                         has_loads_ ? loads_ : nullptr);
     MLFMA_CK(cudaGetLastError());
@@ -2050,12 +2079,13 @@ void DeviceOp::far_l2l_tc(int p, int nr, cudaStream_t s) {
 
 void DeviceOp::drop_graphs() {
     for (int p = 0; p < 2; ++p)
-        for (int t = 0; t < 2; ++t) {
-            if (graph_exec_[p][t]) cudaGraphExecDestroy(graph_exec_[p][t]);
-            if (graph_[p][t]) cudaGraphDestroy(graph_[p][t]);
-            graph_exec_[p][t] = nullptr;
-            graph_[p][t] = nullptr;
-        }
+        for (int t = 0; t < 2; ++t)
+            for (int k = 0; k < 2; ++k) {
+                if (graph_exec_[p][t][k]) cudaGraphExecDestroy(graph_exec_[p][t][k]);
+                if (graph_[p][t][k]) cudaGraphDestroy(graph_[p][t][k]);
+                graph_exec_[p][t][k] = nullptr;
+                graph_[p][t][k] = nullptr;
+            }
 }
 
 std::string DeviceOp::set_tc(int mode) {
@@ -2078,7 +2108,7 @@ std::string DeviceOp::set_near_kernel(int kind) {
     MLFMA_CK(cudaSetDevice(device_));
     MLFMA_CK(cudaStreamSynchronize(stream_));
     near_kernel_ = kind;
-    near_per_sm_ = kind == 2 ? near_direct_occ_ : kind == 1 ? 1 : near_occ_;
+    near_per_sm_ = kind && n_near_quads_ ? near_direct_occ_ : near_occ_;
     set_near_grid(near_per_sm_);
     drop_graphs();
     ++generation_;
@@ -2223,14 +2253,8 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
         if (n_near_tiles_) {
             float bt = 1e30f;
             int bk = near_per_sm_, bkind = near_kernel_;
-            for (int kind : {0, 1, 2})
-                for (int k : kind == 2 ? std::vector<int>{near_direct_occ_ / 2, near_direct_occ_}
-                                       : kind == 1 ? std::vector<int>{1} : [&] {
-                                             std::vector<int> v;
-                                             for (int q = 1; q <= near_occ_; ++q) v.push_back(q);
-                                             return v;
-                                         }()) {
-                    if (k < 1) continue;
+            for (int kind : n_near_quads_ ? std::vector<int>{0, 2} : std::vector<int>{0})
+                for (int k = 1; k <= (kind ? near_direct_occ_ : near_occ_); ++k) {
                     near_kernel_ = kind;
                     set_near_grid(k);
                     const float t = timed(product);

@@ -94,7 +94,7 @@ k_s2m(const DevS2MItem<R>* __restrict__ items, const double2* __restrict__ x) {
 // ------------------------------------------------------------ L2T
 // y_m = sum_e conj(R_m[e]) b_B[e]  (Leaf::evalFarSols, src/fmm/leaf.cpp:257-280;
 // C k is applied when the result is written out).  One block per work item
-// (leaf, run of up to eight sources), two sources per warp with twelve loads in
+// (leaf, run of up to eight sources), two sources per warp with eight loads in
 // flight for each and lane, issued before the leaf's local pattern is staged in
 // shared memory; the sum is widened to complex double on output.
 //
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kL2TThreads, 4)
 k_l2t(const DevL2TItem<R>* __restrict__ items, double2* __restrict__ yfar) {
     chain_wait();
     using C = typename Cx<R>::T;
-    constexpr int RW = kL2TRows, U = 12;
+    constexpr int RW = kL2TRows, U = 8;
     extern __shared__ unsigned char smraw[];
     C* bs = reinterpret_cast<C*>(smraw);
     const DevL2TItem<R> it = items[blockIdx.x];
@@ -133,16 +133,18 @@ k_l2t(const DevL2TItem<R>* __restrict__ items, double2* __restrict__ yfar) {
         __syncthreads();
     }
     const C* b = STAGE ? bs : it.b;
-    C a[RW][2];
+    C a[RW][4];
 #pragma unroll
-    for (int q = 0; q < RW; ++q) a[q][0] = a[q][1] = zero<C>();
+    for (int q = 0; q < RW; ++q)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[q][k] = zero<C>();
     for (int e = lane;;) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (e + 32 * u >= ne) continue;
             const C bv = b[e + 32 * u];
 #pragma unroll
-            for (int q = 0; q < RW; ++q) a[q][u & 1] = CJ ? cjfma(v[q][u], bv, a[q][u & 1]) : cfma(v[q][u], bv, a[q][u & 1]);
+            for (int q = 0; q < RW; ++q) a[q][u & 3] = CJ ? cjfma(v[q][u], bv, a[q][u & 3]) : cfma(v[q][u], bv, a[q][u & 3]);
         }
         e += 32 * U;
         if (e - lane >= ne) break;  // (the whole warp: the sums below shuffle)
@@ -150,7 +152,7 @@ k_l2t(const DevL2TItem<R>* __restrict__ items, double2* __restrict__ yfar) {
     }
 #pragma unroll
     for (int q = 0; q < RW; ++q) {
-        const C acc = warp_sum(cadd(a[q][0], a[q][1]));
+        const C acc = warp_sum(cadd(cadd(a[q][0], a[q][1]), cadd(a[q][2], a[q][3])));
         const int row = warp + q * (kL2TThreads / 32);
         if (lane == 0 && row < it.cnt) yfar[it.src0 + row] = to_d2(acc);
     }

@@ -49,7 +49,7 @@ constexpr int kSymXr = kSymXc + kNearTileCols;
 constexpr int kSymSlot = kSymXr + kNearTileRows;
 constexpr int kSymStageEntries = kSymSlot + (kNearTileRows + kNearTileCols) * 4 / 16;
 constexpr size_t kSymSmemBytes = sizeof(double2) * kSymStageEntries * kSymStages;
-static_assert(kNearTileCols == 64 && kNearTileRows == 64, "k_near_sym maps 64 row and 64 column threads");
+static_assert(kNearTileCols <= 64 && kNearTileRows <= 64, "k_near_sym maps 64 row and 64 column threads");
 static_assert(kNearTileRowsSplit <= 32, "a mode-2 tile's rows are copied by one lane each");
 static_assert((kSymStageEntries * sizeof(double2)) % 16 == 0, "bulk copies need 16-byte aligned stages");
 
@@ -271,277 +271,127 @@ k_near_sym(const DevNearTile* __restrict__ tiles, int ntiles, const double2* __r
     }
 }
 
-// The same tiles, stages and partial slots with one consumer warp per tile:
-// warp w of the kNwConsumers takes the block's tiles w, w + kNwConsumers, ...
-// in its own two stages of the ring (no barrier between consumer warps).
-// Lane l owns tile columns l and l + 32: their x values stay in registers and
-// their column sums accumulate in registers over the whole tile.  Rows go in
-// batches of eight: each lane forms its part of the eight row sums from the
-// same entries it read for the column sums (every entry read from shared
-// memory once), and a reduce-scatter over the warp (three halving exchanges,
-// then two butterflies) leaves row rb + ((l >> 2) & 7) complete in lanes with
-// l & 3 == 0.  A self tile's diagonal counts once, in its row.
-constexpr int kNwConsumers = 4;
-constexpr int kNwThreads = 32 * (1 + kNwConsumers);
-constexpr int kNwStages = 2 * kNwConsumers;
-constexpr size_t kNwSmemBytes = sizeof(double2) * kSymStageEntries * kNwStages;
-
 __device__ __forceinline__ double2 shfl_xor2(double2 v, int m) {
     return make_double2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
 
-__global__ void __launch_bounds__(kNwThreads, 1)
-k_near_warp(const DevNearTile* __restrict__ tiles, int ntiles, const double2* __restrict__ Z,
-            const double2* __restrict__ x, const int* __restrict__ slots, double2* __restrict__ part,
-            int* __restrict__ err) {
-    extern __shared__ __align__(128) unsigned char nw_smem[];
-    double2* stages = reinterpret_cast<double2*>(nw_smem);
-    __shared__ __align__(8) unsigned long long full[kNwStages], empty[kNwStages];
-    __shared__ DevNearTile hdr[kNwStages];
-    __shared__ DevNearTile hbuf[32];  // producer's header batch
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int step = gridDim.x;
-    if (tid == 0) {
-        for (int s = 0; s < kNwStages; ++s) {
-            mbar_init(smem_addr(&full[s]), 1);
-            mbar_init(smem_addr(&empty[s]), 1);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-
-    if (warp == 0) {  // ---- producer warp: as in k_near_sym, over kNwStages stages
-        int it = 0;
-        DevNearTile Tn{};
-        if (blockIdx.x + lane * step < ntiles) Tn = tiles[blockIdx.x + lane * step];
-        for (int t = blockIdx.x; t < ntiles; t += step, ++it) {
-            if ((it & 31) == 0) {
-                __syncwarp();
-                hbuf[lane] = Tn;
-                __syncwarp();
-                const int tb = t + (32 + lane) * step;
-                if (tb < ntiles) Tn = tiles[tb];
-            }
-            const DevNearTile T = hbuf[it & 31];
-            const int s = it % kNwStages;
-            if (it >= kNwStages && !mbar_wait_bounded(smem_addr(&empty[s]), ((it / kNwStages) - 1) & 1)) {
-                if (lane == 0) {
-                    atomicExch(err, 1);
-                    for (int k = 1; k <= kNwStages && k <= it; ++k)  // copies still in flight
-                        mbar_wait_bounded(smem_addr(&full[(it - k) % kNwStages]), ((it - k) / kNwStages) & 1);
-                }
-                return;
-            }
-            double2* st = stages + static_cast<size_t>(s) * kSymStageEntries;
-            int nv = 0, total;
-            long long off = 0;
-            if (T.mode == 2) {
-                if (lane < T.ni) {
-                    const int il = T.i0 + lane;
-                    nv = tile_row_len(T, lane);
-                    off = T.z + (T.kind == 0 ? static_cast<long long>(il) * T.ld : packed_row(il, T.kind)) + T.j0;
-                }
-                total = nv;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-            } else {
-                total = tile_entries(T);
-            }
-            const int nslot = (T.ni + T.nj + 3) & ~3;
-            const uint32_t bytes = static_cast<uint32_t>((total + T.nj + T.ni) * sizeof(double2) + nslot * sizeof(int));
-            const uint32_t b = smem_addr(&full[s]);
-            if (lane == 0) {
-                hdr[s] = T;
-                mbar_arrive_expect_tx(b, bytes);
-            }
-            __syncwarp();
-            if (T.mode == 2) {
-                if (nv > 0) bulk_load(smem_addr(st + lane * T.nj), Z + off, static_cast<uint32_t>(nv * sizeof(double2)), b);
-            } else if (lane == 0) {
-                bulk_load(smem_addr(st), Z + T.z, static_cast<uint32_t>(total * sizeof(double2)), b);
-            }
-            if (lane == 31) bulk_load(smem_addr(st + kSymXc), x + T.c0 + T.j0, static_cast<uint32_t>(T.nj * sizeof(double2)), b);
-            if (lane == 30) bulk_load(smem_addr(st + kSymXr), x + T.r0 + T.i0, static_cast<uint32_t>(T.ni * sizeof(double2)), b);
-            if (lane == 29) bulk_load(smem_addr(st + kSymSlot), slots + T.slot, static_cast<uint32_t>(nslot * sizeof(int)), b);
-        }
-        return;
-    }
-
-    // ---- consumer warps
-    const int cw = warp - 1;
-    const int c0 = lane, c1 = lane + 32;
-    for (int it = cw, t = blockIdx.x + cw * step; t < ntiles; it += kNwConsumers, t += kNwConsumers * step) {
-        const int s = it % kNwStages;
-        const bool ok = mbar_wait_bounded(smem_addr(&full[s]), (it / kNwStages) & 1);
-        if (__any_sync(0xffffffffu, !ok)) {
-            if (lane == 0) atomicExch(err, 1);
-            return;
-        }
-        const DevNearTile T = hdr[s];
-        const double2* zt = stages + static_cast<size_t>(s) * kSymStageEntries;
-        const double2* xr = zt + kSymXr;
-        const int* sl = reinterpret_cast<const int*>(zt + kSymSlot);
-        const double2 xc0 = c0 < T.nj ? zt[kSymXc + c0] : z0();
-        const double2 xc1 = c1 < T.nj ? zt[kSymXc + c1] : z0();
-        // a row's entry at tile column c also enters column c's sum unless it is
-        // on or above a self tile's diagonal
-        const int dcol = T.j0 - T.i0;  // row r, column c is below the diagonal iff r > c + dcol
-        double2 ca0 = z0(), ca1 = z0(), cb0 = z0(), cb1 = z0();
-        for (int rb = 0; rb < T.ni; rb += 8) {
-            double2 p[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int r = rb + j;
-                double2 za = z0(), zb = z0(), xv = z0();
-                if (r < T.ni) {
-                    const int len = tile_row_len(T, r);
-                    const double2* zr = zt + tile_row_start(T, r);
-                    if (c0 < len) za = zr[c0];
-                    if (c1 < len) zb = zr[c1];
-                    xv = xr[r];
-                }
-                p[j] = cfma(za, xc0, cmul(zb, xc1));
-                const bool ia = T.kind == 0 || r > c0 + dcol, ib = T.kind == 0 || r > c1 + dcol;
-                if (j & 1) {
-                    if (ia) cb0 = cfma(za, xv, cb0);
-                    if (ib) cb1 = cfma(zb, xv, cb1);
-                } else {
-                    if (ia) ca0 = cfma(za, xv, ca0);
-                    if (ib) ca1 = cfma(zb, xv, ca1);
-                }
-            }
-            // reduce-scatter of p[0..7] over the warp
-            const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
-            double2 q[4], u[2], w;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double2 send = h4 ? p[k] : p[k + 4];
-                const double2 keep = h4 ? p[k + 4] : p[k];
-                q[k] = cadd(keep, shfl_xor2(send, 16));
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const double2 send = h3 ? q[k] : q[k + 2];
-                const double2 keep = h3 ? q[k + 2] : q[k];
-                u[k] = cadd(keep, shfl_xor2(send, 8));
-            }
-            {
-                const double2 send = h2 ? u[0] : u[1];
-                const double2 keep = h2 ? u[1] : u[0];
-                w = cadd(keep, shfl_xor2(send, 4));
-            }
-            w = cadd(w, shfl_xor2(w, 1));
-            w = cadd(w, shfl_xor2(w, 2));
-            const int r = rb + ((lane >> 2) & 7);
-            if ((lane & 3) == 0 && r < T.ni) {
-                const int slot = sl[r];
-                if (slot >= 0) part[slot] = w;
-            }
-        }
-        if (c0 < T.nj && sl[T.ni + c0] >= 0) part[sl[T.ni + c0]] = cadd(ca0, cb0);
-        if (c1 < T.nj && sl[T.ni + c1] >= 0) part[sl[T.ni + c1]] = cadd(ca1, cb1);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&empty[s]));
-    }
+// One halving exchange: lanes with `hi` keep b, the others a, each added to
+// the partner's copy.
+__device__ __forceinline__ double2 halve(double2 a, double2 b, bool hi, int mask) {
+    const double2 send = hi ? a : b;
+    return cadd(hi ? b : a, shfl_xor2(send, mask));
 }
 
-// The same tiles and partial slots read straight from global memory into
-// registers: no shared-memory stage and no producer warp, so residency is set
-// by registers alone.  Warp w of the grid takes tiles w, w + (warps in the
-// grid), ...; per tile, lane l owns columns l and l + 32 (x values and column
-// sums in registers), rows go in batches of eight (each lane loads its one or
-// two entries of each of the eight rows: coalesced 16-byte loads, all sixteen
-// issued before use) and the row sums are formed by the reduce-scatter of
-// k_near_warp.  A self tile's diagonal counts once, in its row.
+// The same tiles and partial slots with four tiles per warp, straight from
+// global memory into registers: no shared-memory stage, no producer, no barrier.
+// Eight lanes take one tile: lane lc holds its columns lc, lc + 8, ..., their x
+// values and column sums in registers (no reduction over rows), and walks the
+// rows in runs of four; the row sums go through a reduce-scatter over the eight
+// lanes.  A load takes a 128-byte row segment from each of the four tiles, up to
+// 16 of them in flight per lane.  Tiles are grouped by shape (near_quads: all
+// rectangular or all self, by column groups and rows), so that a warp's tiles
+// end together.
+//
+// Bound by memory latency at 12 warps per SM (ncu, 7.8M entries: 50 us cold, 36 %
+// of DRAM, issue 27 %); what it gains on k_near_sym, as fast alone (43 us),
+// is what it leaves to the far-field chain beside it: no shared memory, half the
+// issue slots.  Measured on the way: one tile per warp (lanes 4 x 8 over the
+// tile) spent 950 instructions on 576 entries, 55 us; one instantiation per
+// column count overran the instruction cache, 85 us; entries by cp.async or bulk
+// copies in shared-memory rings, with the fewer warps those leave, 75 and 55 us.
+//
+// A rectangular row is read to the end of the last column group it starts in:
+// past its end lies the next row or tile (kNearPad zeros after the last), which
+// meets an x of zero and a column sum that is not written.  A self tile's
+// diagonal counts once, in its row.
 constexpr int kNdThreads = 128;
+constexpr int kNearPad = 8;
 
-__device__ __forceinline__ long long tile_row_global(const DevNearTile& T, int r) {
-    if (T.mode == 0) return T.z + static_cast<long long>(r) * T.nj;
-    if (T.mode == 1) return T.z + packed_row(T.i0 + r, T.kind) - packed_row(T.i0, T.kind);
-    const int il = T.i0 + r;
-    return T.z + (T.kind == 0 ? static_cast<long long>(il) * T.ld : packed_row(il, T.kind)) + T.j0;
+template <bool SELF>
+__device__ __forceinline__ void near_quad(const DevNearTile& T, const double2* __restrict__ Z,
+                                          const double2* __restrict__ x, const int* __restrict__ slots,
+                                          double2* __restrict__ part) {
+    constexpr int G = kNearQuadCols / 8, RB = 4;
+    const int lc = threadIdx.x & 7;
+    const int nmax = __reduce_max_sync(0xffffffffu, T.ni);
+    const int gmax = __reduce_max_sync(0xffffffffu, (T.nj + 7) >> 3);
+    const int* sl = slots + T.slot;
+    const double2* xr = x + T.r0 + T.i0;
+    const double2* xc0 = x + T.c0 + T.j0 + lc;
+    // row r of a rectangular tile: zb + r stride
+    const int stride = T.mode == 0 ? T.nj : T.ld;
+    const double2* zb = Z + T.z + lc;
+    if (!SELF && T.mode == 2) zb += static_cast<long long>(T.i0) * T.ld + T.j0;
+    double2 xc[G], ca[G];
+    int cslot[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+        const bool in = lc + 8 * j < T.nj;
+        xc[j] = in ? xc0[8 * j] : z0();
+        cslot[j] = in ? sl[T.ni + lc + 8 * j] : -1;
+        ca[j] = z0();
+    }
+    const int dcol = T.j0 - T.i0;  // self: row r, column c is below the diagonal iff r > c + dcol
+    // the row of a run this lane ends up with
+    const int ro = (lc >> 2) << 1 | ((lc >> 1) & 1);
+    for (int rb = 0; rb < nmax; rb += RB) {
+        double2 z[RB][G], xv[RB], p[RB];
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+            const int r = rb + i;
+            const bool in = r < T.ni;
+            xv[i] = in ? xr[r] : z0();
+            int len = in ? T.nj : 0;
+            const double2* zr = zb + r * stride;
+            if (SELF) {
+                len = in ? tile_row_len(T, r) : 0;
+                const int il = T.i0 + r;  // mode 1: packed rows; 2: a column range of them
+                zr = zb + (T.mode == 1 ? packed_row(il, T.kind) - packed_row(T.i0, T.kind)
+                                       : packed_row(il, T.kind) + T.j0);
+            }
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                z[i][j] = z0();
+                if (j < gmax && (SELF ? lc + 8 * j : 8 * j) < len) z[i][j] = __ldcs(zr + 8 * j);
+            }
+        }
+        const int rslot = (lc & 1) == 0 && rb + ro < T.ni ? sl[rb + ro] : -1;
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+            p[i] = z0();
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if (j >= gmax) break;
+                p[i] = cfma(z[i][j], xc[j], p[i]);
+                if (!SELF || rb + i > lc + 8 * j + dcol) ca[j] = cfma(z[i][j], xv[i], ca[j]);
+            }
+        }
+        const double2 q0 = halve(p[0], p[2], lc & 4, 4), q1 = halve(p[1], p[3], lc & 4, 4);
+        double2 w = halve(q0, q1, lc & 2, 2);
+        w = cadd(w, shfl_xor2(w, 1));
+        if (rslot >= 0) part[rslot] = w;
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+        if (cslot[j] >= 0) part[cslot[j]] = ca[j];
 }
 
-__global__ void __launch_bounds__(kNdThreads)
-k_near_direct(const DevNearTile* __restrict__ tiles, int ntiles, const double2* __restrict__ Z,
+__global__ void __launch_bounds__(kNdThreads, 3)
+k_near_direct(const DevNearTile* __restrict__ quads, int nquads, const double2* __restrict__ Z,
               const double2* __restrict__ x, const int* __restrict__ slots, double2* __restrict__ part) {
-    const int lane = threadIdx.x & 31;
+    const int g = (threadIdx.x & 31) >> 3;
     const int nwarps = gridDim.x * (kNdThreads / 32);
-    const int c0 = lane, c1 = lane + 32;
-    for (int t = blockIdx.x * (kNdThreads / 32) + (threadIdx.x >> 5); t < ntiles; t += nwarps) {
-        const DevNearTile T = tiles[t];
-        const double2* xr = x + T.r0 + T.i0;
-        const int* sl = slots + T.slot;
-        const double2 xc0 = c0 < T.nj ? x[T.c0 + T.j0 + c0] : z0();
-        const double2 xc1 = c1 < T.nj ? x[T.c0 + T.j0 + c1] : z0();
-        const int dcol = T.j0 - T.i0;  // row r, column c is below the diagonal iff r > c + dcol
-        double2 ca0 = z0(), ca1 = z0(), cb0 = z0(), cb1 = z0();
-        for (int rb = 0; rb < T.ni; rb += 8) {
-            double2 za[8], zb[8], xv[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int r = rb + j;
-                za[j] = z0();
-                zb[j] = z0();
-                xv[j] = z0();
-                if (r < T.ni) {
-                    const int len = tile_row_len(T, r);
-                    const double2* zr = Z + tile_row_global(T, r);
-                    if (c0 < len) za[j] = __ldcs(zr + c0);
-                    if (c1 < len) zb[j] = __ldcs(zr + c1);
-                    xv[j] = xr[r];
-                }
-            }
-            double2 p[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int r = rb + j;
-                p[j] = cfma(za[j], xc0, cmul(zb[j], xc1));
-                const bool ia = T.kind == 0 || r > c0 + dcol, ib = T.kind == 0 || r > c1 + dcol;
-                if (j & 1) {
-                    if (ia) cb0 = cfma(za[j], xv[j], cb0);
-                    if (ib) cb1 = cfma(zb[j], xv[j], cb1);
-                } else {
-                    if (ia) ca0 = cfma(za[j], xv[j], ca0);
-                    if (ib) ca1 = cfma(zb[j], xv[j], ca1);
-                }
-            }
-            // reduce-scatter of p[0..7] over the warp (as in k_near_warp)
-            const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
-            double2 q[4], u[2], w;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double2 send = h4 ? p[k] : p[k + 4];
-                const double2 keep = h4 ? p[k + 4] : p[k];
-                q[k] = cadd(keep, shfl_xor2(send, 16));
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const double2 send = h3 ? q[k] : q[k + 2];
-                const double2 keep = h3 ? q[k + 2] : q[k];
-                u[k] = cadd(keep, shfl_xor2(send, 8));
-            }
-            {
-                const double2 send = h2 ? u[0] : u[1];
-                const double2 keep = h2 ? u[1] : u[0];
-                w = cadd(keep, shfl_xor2(send, 4));
-            }
-            w = cadd(w, shfl_xor2(w, 1));
-            w = cadd(w, shfl_xor2(w, 2));
-            const int r = rb + ((lane >> 2) & 7);
-            if ((lane & 3) == 0 && r < T.ni) {
-                const int slot = sl[r];
-                if (slot >= 0) part[slot] = w;
-            }
-        }
-        if (c0 < T.nj) {
-            const int slot = sl[T.ni + c0];
-            if (slot >= 0) part[slot] = cadd(ca0, cb0);
-        }
-        if (c1 < T.nj) {
-            const int slot = sl[T.ni + c1];
-            if (slot >= 0) part[slot] = cadd(ca1, cb1);
-        }
+    int q = blockIdx.x * (kNdThreads / 32) + (threadIdx.x >> 5);
+    if (q >= nquads) return;
+    DevNearTile T = quads[4 * static_cast<size_t>(q) + g];
+    while (true) {
+        const int qn = q + nwarps;
+        const DevNearTile Tn = quads[4 * static_cast<size_t>(min(qn, nquads - 1)) + g];
+        if (T.kind != 0) near_quad<true>(T, Z, x, slots, part);  // (a warp's tiles are of one kind)
+        else near_quad<false>(T, Z, x, slots, part);
+        if (qn >= nquads) break;
+        T = Tn;
+        q = qn;
     }
 }
 

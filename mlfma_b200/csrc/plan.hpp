@@ -135,6 +135,23 @@ struct NearTile {
     int mode;             // layout, above
 };
 
+// A near field of up to kNearQuadEntries stored entries is also cut into tiles
+// of at most kNearQuadCols columns, applied four to a warp (k_near_direct); a
+// larger one keeps k_near_sym's alone.  The narrow tiles write more partial sums,
+// which cost little while they stay in the L2 (about 0.08 per entry: 36M entries
+// 46 MB; 133M entries 170 MB).  One B200, whole products, k_near_sym and
+// k_near_direct: 7.8M entries 197 and 184 us FP64, 133 and 112 us complex-float
+// far field; 36M entries 511 and 486 us (complex float); 133M entries 2,008 and
+// 2,080 us.
+constexpr int kNearQuadCols = 32;
+constexpr long long kNearQuadEntries = 48ll << 20;
+struct NearTiling {
+    std::vector<NearTile> tiles;
+    int parts = 0;                // partial sums the tiles write
+    std::vector<int> slot;        // per tile, padded to 4: slot of each partial
+    std::vector<int> red_ptr;     // [n + 1]: target t's partials are slots ptr[t]..ptr[t+1]
+};
+
 struct FarLeaf {
     int level, box, src0, nsrc;
     long long pat_off;  // offset in units of (direction, 2 components)
@@ -176,6 +193,7 @@ struct Plan {
     int near_parts = 0;                   // partial sums the tiles write
     std::vector<int> near_slot;           // per tile, padded to 4: slot of each partial
     std::vector<int> near_red_ptr;        // [n + 1]: target t's partials are slots ptr[t]..ptr[t+1]
+    NearTiling near_quads;                // the same blocks in tiles of at most kNearQuadCols columns, if any
     std::vector<NearRow> near_rows;       // both orientations, per leaf (many-rhs storage)
     std::vector<int> near_cols;
     long long near_row_entries = 0;
@@ -203,6 +221,7 @@ private:
     void build_levels();
     void build_far_plan();
     void build_near_plan();
+    void tile_near_blocks(int cols, NearTiling& out) const;
 };
 
 // The 26 neighbour directions in the reference's order (FMM::Dir,
