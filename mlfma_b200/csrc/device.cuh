@@ -77,7 +77,28 @@ struct DevTransT {
     //                                direction that tap reads.
     const typename Cx<R>::T* fold_up;
     const typename Cx<R>::T* fold_dn;
+    // Groups of neighbouring outputs (k_m2m_w, k_l2l_w; null where the unions of
+    // their taps do not fit): the taps of each union in order, [group][kWinTapsUp]
+    // (source row; bit 0 reflected, bit 1 + j: row j has it) and
+    // [side][group][kWinTapsDn] (parent column, mask of columns); their counts; weights [..][tap][output], zero where
+    // the output has no such tap; and, complex float, the L2L's with the shift
+    // folded in as fold_dn, [oct][ith][side][group][tap][kWinCols].
+    const int2* win_up;
+    const int* win_up_n;
+    const R* win_up_w;
+    const int2* win_dn;
+    const int* win_dn_n;
+    const R* win_dn_w;
+    // theta pass of the L2L: groups of kWinCols child rows, [group][kWinTapsTh]
+    // (parent row; bit 0 reflected, bit 1 + i: row i has it), as above
+    const int2* win_th;
+    const int* win_th_n;
+    const R* win_th_w;
+    const typename Cx<R>::T* fold_dnw;
 };
+
+constexpr int kWinRows = 4, kWinTapsUp = 10;
+constexpr int kWinCols = 3, kWinTapsDn = 16, kWinTapsTh = 20;
 
 struct DevFarLeaf {
     int level, box, src0, nsrc;
@@ -353,6 +374,9 @@ public:
 private:
     template <class T> T* alloc(size_t count);
     template <class T> T* upload(const std::vector<T>& v);
+    template <class R>
+    void build_windows(const Transition& T, const Level& PL, const Level& CL, int wd, const std::vector<cplx>& fd,
+                       DevTransT<R>& d);
     template <class R> std::string setup_far(const Plan& plan, FarField<R>& F, const double2* pat64);
     template <class R, bool TR> void run_far_t(FarField<R>& F, const double2* xt, cudaStream_t s, int stage);
     template <class R, bool TR> void run_far_overlap_t(FarField<R>& F, const double2* xt, cudaStream_t s,
@@ -492,8 +516,7 @@ private:
     std::vector<DevM2LGroup> h_groups_;
     std::vector<short> h_cand_off_;        // [candidate][kMaxGroup] offset ids (-1: none)
     int* m2l_cand_src_ = nullptr;
-    int2* m2l_items_m_ = nullptr;
-    int n_m2l_items_m_ = 0;
+    int m2l_group_first_[kMaxLevels] = {}, m2l_group_count_[kMaxLevels] = {};  // groups of each level
     // Tensor-core interpolation (complex-float far field), per transition.
     std::vector<TcTrans> tc_;
     float* tc_scratch_ = nullptr;       // intermediate of the two passes of a stage

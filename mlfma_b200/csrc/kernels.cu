@@ -123,6 +123,7 @@ template <> double2 host_c<double2>(const cplx& v) { return make_double2(v.real(
 template <> float2 host_c<float2>(const cplx& v) {
     return make_float2(static_cast<float>(v.real()), static_cast<float>(v.imag()));
 }
+template <class C> C zero_host() { return C{0, 0}; }
 template <class C> std::vector<C> conv_c(const std::vector<cplx>& v) {
     std::vector<C> o(v.size());
     for (size_t i = 0; i < v.size(); ++i) o[i] = host_c<C>(v[i]);
@@ -392,6 +393,122 @@ std::string DeviceOp::build_transl_device(const Level& L, double2* t) {
 }
 
 // Far-field arrays in precision R (levels, transitions, patterns).
+// The windowed stencils of one transition (k_m2m_w, k_l2l_w); fd: the folded
+// weights of dn_ph.  Left null where a union of taps is too wide.
+template <class R>
+void DeviceOp::build_windows(const Transition& T, const Level& PL, const Level& CL, int wd, const std::vector<cplx>& fd,
+                             DevTransT<R>& d) {
+    using C = typename Cx<R>::T;
+    constexpr bool f64 = std::is_same<R, double>::value;
+    if constexpr (f64) {  // M2M: groups of parent theta rows; a tap's place is its index before the pole reflection
+        const int mth = CL.nth, ng = (PL.nth + kWinRows - 1) / kWinRows;
+        std::vector<int2> win(static_cast<size_t>(ng) * kWinTapsUp, make_int2(0, 0));
+        std::vector<R> wt(win.size() * kWinRows, R(0));
+        std::vector<int> cnt(ng, 0);
+        bool fits = true;
+        auto place = [&](int q) {
+            const int s = T.up_th.src[q];
+            return !T.up_th.refl[q] ? s : s < mth / 2 ? -s - 1 : 2 * mth - 1 - s;
+        };
+        for (int g = 0; g < ng && fits; ++g) {
+            const int first = g * kWinRows, rows = std::min(kWinRows, PL.nth - first);
+            std::vector<std::pair<int, int>> u;  // (place, a tap with it)
+            for (int q = T.up_th.ptr[first]; q < T.up_th.ptr[first + rows]; ++q) u.emplace_back(place(q), q);
+            std::sort(u.begin(), u.end());
+            u.erase(std::unique(u.begin(), u.end(), [](const auto& a, const auto& b) { return a.first == b.first; }),
+                    u.end());
+            fits = u.size() <= static_cast<size_t>(kWinTapsUp);
+            if (!fits) break;
+            cnt[g] = static_cast<int>(u.size());
+            for (size_t t = 0; t < u.size(); ++t)
+                win[g * kWinTapsUp + t] = make_int2(T.up_th.src[u[t].second], T.up_th.refl[u[t].second]);
+            for (int j = 0; j < rows; ++j)
+                for (int q = T.up_th.ptr[first + j]; q < T.up_th.ptr[first + j + 1]; ++q) {
+                    size_t t = 0;
+                    while (u[t].first != place(q)) ++t;
+                    win[g * kWinTapsUp + t].y |= 2 << j;
+                    wt[(g * kWinTapsUp + t) * kWinRows + j] = static_cast<R>(T.up_th.refl[q] ? -T.up_th.coef[q] : T.up_th.coef[q]);
+                }
+        }
+        if (fits) {
+            d.win_up = upload(win);
+            d.win_up_n = upload(cnt);
+            d.win_up_w = upload(wt);
+        }
+    }
+    // L2L: groups of child phi columns and their partners half a turn on
+    const int cph = CL.nph, half = cph / 2, ng = (half + kWinCols - 1) / kWinCols;
+    std::vector<int2> win(static_cast<size_t>(2) * ng * kWinTapsDn, make_int2(0, 0));
+    std::vector<R> wt(win.size() * kWinCols, R(0));
+    std::vector<int> cnt(2 * ng, 0);
+    std::vector<C> f(f64 ? 0 : static_cast<size_t>(8) * PL.nth * win.size() * kWinCols, zero_host<C>());
+    for (int sg = 0; sg < 2 * ng; ++sg) {
+        const int first = (sg % ng) * kWinCols, cols = std::min(kWinCols, half - first), turn = sg / ng * half;
+        std::vector<int> u;
+        for (int q = T.dn_ph.ptr[first + turn]; q < T.dn_ph.ptr[first + turn + cols]; ++q) u.push_back(T.dn_ph.src[q]);
+        std::sort(u.begin(), u.end());
+        u.erase(std::unique(u.begin(), u.end()), u.end());
+        if (u.size() > static_cast<size_t>(kWinTapsDn)) return;
+        cnt[sg] = static_cast<int>(u.size());
+        for (size_t t = 0; t < u.size(); ++t) win[sg * kWinTapsDn + t].x = u[t];
+        for (int j = 0; j < cols; ++j) {
+            const int c = first + turn + j;
+            int last = -1;
+            for (int q = T.dn_ph.ptr[c]; q < T.dn_ph.ptr[c + 1]; ++q) {
+                const int t = static_cast<int>(std::lower_bound(u.begin(), u.end(), T.dn_ph.src[q]) - u.begin());
+                if (t <= last) return;  // (a column's taps are in order, each once)
+                last = t;
+                win[sg * kWinTapsDn + t].y |= 1 << j;
+                wt[(sg * kWinTapsDn + t) * kWinCols + j] = static_cast<R>(T.dn_ph.refl[q] ? -T.dn_ph.coef[q] : T.dn_ph.coef[q]);
+                if constexpr (!f64)
+                    for (int oct = 0; oct < 8; ++oct)
+                        for (int ith = 0; ith < PL.nth; ++ith)
+                            f[(((static_cast<size_t>(oct) * PL.nth + ith) * (2 * ng) + sg) * kWinTapsDn + t) * kWinCols + j] =
+                                host_c<C>(fd[((static_cast<size_t>(oct) * PL.nth + ith) * cph + c) * wd + q - T.dn_ph.ptr[c]]);
+            }
+        }
+    }
+    // its theta pass: groups of child rows; at one parent row a row's taps are the
+    // reflection at the north pole, the direct one, the reflection at the south pole
+    const int cth = CL.nth, ngt = (cth + kWinCols - 1) / kWinCols;
+    std::vector<int2> wth(static_cast<size_t>(ngt) * kWinTapsTh, make_int2(0, 0));
+    std::vector<R> wthw(wth.size() * kWinCols, R(0));
+    std::vector<int> nth(ngt, 0);
+    for (int g = 0; g < ngt; ++g) {
+        const int first = g * kWinCols, rows = std::min(kWinCols, cth - first);
+        auto key = [&](int row, int q) {
+            return 3 * T.dn_th.src[q] + (!T.dn_th.refl[q] ? 1 : row < cth / 2 ? 0 : 2);
+        };
+        std::vector<std::pair<int, int>> u;  // (key, a tap with it)
+        for (int i = 0; i < rows; ++i)
+            for (int q = T.dn_th.ptr[first + i]; q < T.dn_th.ptr[first + i + 1]; ++q) u.emplace_back(key(first + i, q), q);
+        std::sort(u.begin(), u.end());
+        u.erase(std::unique(u.begin(), u.end(), [](const auto& a, const auto& b) { return a.first == b.first; }), u.end());
+        if (u.size() > static_cast<size_t>(kWinTapsTh)) return;
+        nth[g] = static_cast<int>(u.size());
+        for (size_t t = 0; t < u.size(); ++t)
+            wth[g * kWinTapsTh + t] = make_int2(T.dn_th.src[u[t].second], T.dn_th.refl[u[t].second]);
+        for (int i = 0; i < rows; ++i) {
+            int last = -1;
+            for (int q = T.dn_th.ptr[first + i]; q < T.dn_th.ptr[first + i + 1]; ++q) {
+                int t = 0;
+                while (u[t].first != key(first + i, q)) ++t;
+                if (t <= last) return;  // (a row's taps are in order, each once)
+                last = t;
+                wth[g * kWinTapsTh + t].y |= 2 << i;
+                wthw[(g * kWinTapsTh + t) * kWinCols + i] = static_cast<R>(T.dn_th.refl[q] ? -T.dn_th.coef[q] : T.dn_th.coef[q]);
+            }
+        }
+    }
+    d.win_th = upload(wth);
+    d.win_th_n = upload(nth);
+    d.win_th_w = upload(wthw);
+    d.win_dn = upload(win);
+    d.win_dn_n = upload(cnt);
+    d.win_dn_w = upload(wt);
+    if (!f64) d.fold_dnw = upload(f);
+}
+
 template <class R>
 std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2* pat64) {
     using C = typename Cx<R>::T;
@@ -476,6 +593,8 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         d.plevel = p;
         d.npar = static_cast<int>(T.par_box.size());
         d.fold_up = d.fold_dn = nullptr;
+        d.win_up = nullptr;
+        d.win_dn = nullptr;
         if (max_rhs_ > 1) {
             const Level& PL = plan.levels[p];
             const Level& CL = plan.levels[p + 1];
@@ -507,6 +626,7 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
                         }
             d.fold_up = upload(conv_c<C>(fu));
             d.fold_dn = upload(conv_c<C>(fd));
+            build_windows(T, PL, CL, wd, fd, d);
         }
         d.par_box = upload(T.par_box);
         d.par_ilist = upload(T.par_ilist);
@@ -635,6 +755,9 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
             if (e != cudaSuccess) return e;
             return cudaFuncSetAttribute(fn, attr, dev_smem - static_cast<int>(fa.sharedSizeBytes));
         };
+        MLFMA_CK(dyn(reinterpret_cast<const void*>(k_m2m_w<6>)));
+        MLFMA_CK(dyn(reinterpret_cast<const void*>(k_l2l_w<R, 1>)));
+        if constexpr (std::is_same<R, float>::value) MLFMA_CK(dyn(reinterpret_cast<const void*>(k_l2l_w<R, 2>)));
         MLFMA_CK(dyn(reinterpret_cast<const void*>(k_m2m_m<R, 2, 8>)));
         MLFMA_CK(dyn(reinterpret_cast<const void*>(k_m2m_m<R, 4, 8>)));
         MLFMA_CK(dyn(reinterpret_cast<const void*>(k_m2m_m<R, 6, 8>)));
@@ -1644,11 +1767,11 @@ std::string DeviceOp::setup_multi(const Plan& plan) {
     n_near_items_m_ = static_cast<int>(nit.size());
     near_items_m_ = upload(nit);
     // Many-rhs M2L: weighted transfer values per (group, direction, candidate,
-    // target), and direction-major items (the blocks in flight together all
-    // read the patterns of one direction, 2 KB per box at 64 rhs, which stay
-    // in L2 for every group that needs them).
+    // target).  A level's groups are contiguous; the kernel walks them
+    // direction-major (the blocks in flight together all read the patterns of
+    // one run of directions, 2 KB per box and direction at 64 rhs, which stay in
+    // L2 for every group that needs them).
     std::vector<cplx> t8;
-    std::vector<int2> items;
     for (int l = lmin_; l <= lmax_; ++l) {
         const Level& L = plan.levels[l];
         std::vector<int> gl;
@@ -1667,14 +1790,12 @@ std::string DeviceOp::setup_multi(const Plan& plan) {
                                 L.transl[static_cast<size_t>(o) * L.ndir + d] * L.m2l_w[d];
                     }
         }
-        for (int d = 0; d < L.ndir; ++d)
-            for (int gi : gl) items.push_back(make_int2(gi, d));
+        m2l_group_first_[l] = gl.empty() ? 0 : gl.front();
+        m2l_group_count_[l] = static_cast<int>(gl.size());
     }
     MLFMA_CK(h2d_landed(m2l_groups_, h_groups_.data(), sizeof(DevM2LGroup) * h_groups_.size()));
     f64_.m2l_t8 = upload(conv_c<double2>(t8));
     if (precision_ != kFp64) f32_.m2l_t8 = upload(conv_c<float2>(t8));
-    n_m2l_items_m_ = static_cast<int>(items.size());
-    m2l_items_m_ = upload(items);
     return {};
 }
 
@@ -1739,13 +1860,25 @@ std::string DeviceOp::build_m2l_groups(const Plan& plan) {
     return {};
 }
 
+// f(TN) for the least TN = 1..4 with 16 TN >= nr: the width of the GEMM tiles.
+template <class F>
+void by_columns(int nr, F f) {
+    if (nr <= 16) f(std::integral_constant<int, 1>());
+    else if (nr <= 32) f(std::integral_constant<int, 2>());
+    else if (nr <= 48) f(std::integral_constant<int, 3>());
+    else f(std::integral_constant<int, 4>());
+}
+
 // stage: -1 all, 0 S2M, 1 M2M, 2 M2L, 3 L2L, 4 L2T.
 template <class R>
 void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage) {
     using C = typename Cx<R>::T;
     if (n_leaves_ == 0) return;
     if ((stage < 0 || stage == 0) && n_s2m_items_m_)
-        k_s2m_m<R><<<n_s2m_items_m_, kGemmThreads, 0, s>>>(F.lv_dev, s2m_items_m_, leaves_, F.pat, xtm_, nr);
+        by_columns(nr, [&](auto tn) {
+            k_s2m_m<R, decltype(tn)::value>
+                <<<n_s2m_items_m_, kGemmThreads, 0, s>>>(F.lv_dev, s2m_items_m_, leaves_, F.pat, xtm_, nr);
+        });
     const bool tc_up = std::is_same<R, float>::value && (tc_mode_ & 2);
     const bool tc_dn = std::is_same<R, float>::value && (tc_mode_ & 8);
     if ((stage < 0 || stage == 1) && tc_up)
@@ -1753,6 +1886,15 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
     if ((stage < 0 || stage == 1) && !tc_up)
         for (int p = lmax_ - 1; p >= lmin_; --p) {
             if (npar_[p] == 0) continue;
+            if constexpr (std::is_same<R, double>::value) {
+                const size_t wsm = sizeof(C) * nph_[p + 1] * kWinRows * 32;
+                if (F.trans[p].win_up && up_w_[p] == 6 && wsm <= kWinSmem && precision_ == kFp64) {
+                    const int ng = (nth_[p] + kWinRows - 1) / kWinRows;
+                    k_m2m_w<6><<<static_cast<unsigned>(npar_[p]) * ng * ((nr + 15) / 16), kInterpThreads, wsm, s>>>(
+                        F.lv_dev, F.trans[p], nr, ng);
+                    continue;
+                }
+            }
             constexpr int rc = 16 * m2m_rpl<R>();
             const int rows_fast = m_m2m_rows_fast_ < 0 ? (m2m_rows_fast<R>() ? 1 : 0) : m_m2m_rows_fast_;
             const dim3 grid = rows_fast ? dim3(nth_[p], (nr + rc - 1) / rc, npar_[p])
@@ -1772,10 +1914,15 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
             }
 #undef MLFMA_M2M_M
         }
-    if ((stage < 0 || stage == 2) && n_m2l_items_m_) {
-        const int threads = std::min(kM2LmThreads, ((2 * nr + 31) / 32) * 32);
-        k_m2l_m<R><<<n_m2l_items_m_, threads, 0, s>>>(F.lv_dev, m2l_items_m_, m2l_groups_, m2l_cand_src_,
-                                                      F.m2l_t8, nr, ref_compat_ ? 0 : 1);
+    if (stage < 0 || stage == 2) {
+        const int D = std::max(1, std::min(kM2LmDirs, kM2LmThreads / (2 * nr)));
+        const int threads = std::min(kM2LmThreads, ((2 * nr * D + 31) / 32) * 32);
+        const size_t smem = sizeof(C) * D * kCandChunk * kMaxGroup;
+        for (int l = lmin_; l <= lmax_; ++l)
+            if (m2l_group_count_[l])
+                k_m2l_m<R><<<m2l_group_count_[l] * ((ndir_[l] + D - 1) / D), threads, smem, s>>>(
+                    F.lv_dev, m2l_groups_ + m2l_group_first_[l], m2l_group_count_[l], m2l_cand_src_, F.m2l_t8, nr, D,
+                    ref_compat_ ? 0 : 1);
     }
     if ((stage < 0 || stage == 3) && tc_dn)
         for (int p = lmin_; p < lmax_; ++p) far_l2l_tc(p, nr, s);
@@ -1783,6 +1930,26 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
         for (int p = lmin_; p < lmax_; ++p) {
             const int g = n_l2l_pairs_[p];
             if (!g) continue;
+            // complex float: two right-hand sides a lane (each weight read serves
+            // both) where the tile still leaves room for two blocks on an SM
+            auto wsm = [&](int rpl) {
+                return sizeof(C) * nth_[p] * 2 * kWinCols * 32 * rpl +
+                       static_cast<size_t>((nth_[p + 1] + kWinCols - 1) / kWinCols) * kWinTapsTh *
+                           (kWinCols * sizeof(R) + sizeof(int2));
+            };
+            if (F.trans[p].win_dn && wsm(1) <= kWinSmem &&
+                (std::is_same<R, float>::value || precision_ == kFp64)) {
+                const int ng = (nph_[p + 1] / 2 + kWinCols - 1) / kWinCols;
+                if constexpr (std::is_same<R, float>::value)
+                    if (nr > 16 && wsm(2) <= kWinSmem) {
+                        k_l2l_w<R, 2><<<dim3(g, ng, (nr + 31) / 32), kInterpThreads, wsm(2), s>>>(F.lv_dev, F.trans[p],
+                                                                                                 l2l_pairs_[p], nr);
+                        continue;
+                    }
+                k_l2l_w<R, 1><<<dim3(g, ng, (nr + 15) / 16), kInterpThreads, wsm(1), s>>>(F.lv_dev, F.trans[p],
+                                                                                         l2l_pairs_[p], nr);
+                continue;
+            }
             const int pairs = m_l2l_pairs_ > 0 ? m_l2l_pairs_ : l2l_pairs<R>();
             const dim3 grid(g, (nph_[p + 1] / 2 + pairs - 1) / pairs, (nr + kRc - 1) / kRc);
             const size_t smem = static_cast<size_t>(nth_[p]) * 2 * pairs * 64 * sizeof(C) +
@@ -1801,7 +1968,10 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
 #undef MLFMA_L2L_M
         }
     if ((stage < 0 || stage == 4) && n_l2t_items_m_)
-        k_l2t_m<R><<<n_l2t_items_m_, kGemmThreads, 0, s>>>(F.lv_dev, l2t_items_m_, leaves_, F.pat, yfarm_, nr);
+        by_columns(nr, [&](auto tn) {
+            k_l2t_m<R, decltype(tn)::value>
+                <<<n_l2t_items_m_, kGemmThreads, 0, s>>>(F.lv_dev, l2t_items_m_, leaves_, F.pat, yfarm_, nr);
+        });
 }
 
 void DeviceOp::run_far_multi(int nr, cudaStream_t s, int stage, int prec) {
@@ -1811,8 +1981,10 @@ void DeviceOp::run_far_multi(int nr, cudaStream_t s, int stage, int prec) {
 
 void DeviceOp::run_near_multi(int nr, cudaStream_t s) {
     if (n_near_items_m_ == 0) return;
-    k_near_m<<<n_near_items_m_, kGemmThreads, 0, s>>>(near_rows_, near_items_m_, near_z_, near_cols_, xtm_, ynearm_,
-                                                       nr);
+    by_columns(nr, [&](auto tn) {
+        k_near_m<decltype(tn)::value><<<n_near_items_m_, kGemmThreads, 0, s>>>(near_rows_, near_items_m_, near_z_,
+                                                                               near_cols_, xtm_, ynearm_, nr);
+    });
 }
 
 // xtm_ -> (yfarm_, ynearm_): near field on the side stream, far field on s.
