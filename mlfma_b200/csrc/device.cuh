@@ -386,6 +386,7 @@ private:
     // is a kernel of the chain, and the only one this launch depends on)
     template <class R, bool TR> void far_s2m(FarField<R>& F, const double2* xt, cudaStream_t s);
     template <class R, bool TR> void far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl = false);
+    template <class R, bool TR> void far_m2l_boxes(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl);
     template <class R, bool TR> void far_m2l(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl = false);
     template <class R, bool TR> void far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl = false);
     template <class R, bool TR> void far_l2t(FarField<R>& F, cudaStream_t s, bool pdl = false);

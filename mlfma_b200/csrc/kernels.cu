@@ -1198,21 +1198,32 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     }
 }
 
-// M2L of levels lo..hi (their items are contiguous, level by level).
+// M2L of levels lo..hi box by box (their items are contiguous, level by level).
+// Blocks hold as many warps as the widest of the levels' direction runs fills:
+// 162 directions are two runs of 81, three warps and not four.
+template <class R, bool TR>
+void DeviceOp::far_m2l_boxes(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl) {
+    const int first = m2l_first_[lo], count = m2l_first_[hi] + m2l_count_[hi] - first;
+    if (count <= 0) return;
+    int widest = 1;
+    for (int l = lo; l <= hi; ++l) {
+        const int nchunk = (ndir_[l] + m2l_chunk_ - 1) / m2l_chunk_;
+        widest = std::max(widest, (ndir_[l] + nchunk - 1) / nchunk);
+    }
+    launch_k(pdl, m2l_staged_ ? k_m2l_staged<R, TR> : k_m2l<R, TR>, count, (widest + 31) / 32 * 32, 0, s, F.lv_dev,
+             m2l_items_ + first, ref_compat_ ? 0 : 1);
+}
+
+// M2L of levels lo..hi.
 template <class R, bool TR>
 void DeviceOp::far_m2l(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl) {
     if (lo > hi) return;
-    const int first = m2l_first_[lo];
-    const int count = m2l_first_[hi] + m2l_count_[hi] - first;
-    if (count <= 0) return;
     if constexpr (std::is_same<R, double>::value) {
         if (m2l_staged_) {
             for (int l = lo; l <= hi; ++l) {
                 const int nf = m2l_fam_count_[l];
                 if (!nf) {  // a level below the families' threshold
-                    if (m2l_count_[l])
-                        launch_k(pdl, k_m2l_staged<R, TR>, m2l_count_[l], 128, 0, s, F.lv_dev,
-                                 m2l_items_ + m2l_first_[l], ref_compat_ ? 0 : 1);
+                    far_m2l_boxes<R, TR>(F, l, l, s, pdl);
                     pdl = pdl && !m2l_count_[l];
                     continue;
                 }
@@ -1230,8 +1241,7 @@ void DeviceOp::far_m2l(FarField<R>& F, int lo, int hi, cudaStream_t s, bool pdl)
             return;
         }
     }
-    launch_k(pdl, m2l_staged_ ? k_m2l_staged<R, TR> : k_m2l<R, TR>, count, 128, 0, s, F.lv_dev, m2l_items_ + first,
-             ref_compat_ ? 0 : 1);
+    far_m2l_boxes<R, TR>(F, lo, hi, s, pdl);
 }
 
 template <class R, bool TR>

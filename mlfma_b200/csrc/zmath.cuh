@@ -67,6 +67,26 @@ __device__ __forceinline__ void atomic_add_z(double2* p, double2 v) {
 __device__ __forceinline__ double2 ldg_stream(const double2* p) { return __ldcs(p); }
 __device__ __forceinline__ float2 ldg_stream(const float2* p) { return __ldcs(p); }
 
+// The two components of a direction (p: an even element of a pattern), one
+// 16-byte access in complex float: element by element a warp's 8-byte accesses
+// are 16 bytes apart and take twice the wavefronts.
+__device__ __forceinline__ void load_pair(const double2* p, double2& a, double2& b) {
+    a = p[0];
+    b = p[1];
+}
+__device__ __forceinline__ void load_pair(const float2* p, float2& a, float2& b) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = make_float2(v.x, v.y);
+    b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void store_pair(double2* p, double2 a, double2 b) {
+    p[0] = a;
+    p[1] = b;
+}
+__device__ __forceinline__ void store_pair(float2* p, float2 a, float2 b) {
+    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
+}
+
 // Conversions between the far-field type and complex double.
 template <class C> __device__ __forceinline__ C from_d2(double2 v);
 template <> __device__ __forceinline__ double2 from_d2<double2>(double2 v) { return v; }
