@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cmath>
 #include <deque>
+#include <future>
 #include <thread>
 #include <functional>
 #include <limits>
@@ -946,14 +947,17 @@ void Plan::build_near_plan() {
         add(A.src_begin, A.src_count, A.src_begin, A.src_count, 1);
     }
 
+    // (the quads' tiles on another thread, beside the wide ones and the block rows)
+    near_quads = NearTiling{};
+    std::future<void> quads;
+    if (near_entries <= kNearQuadEntries)
+        quads = std::async(std::launch::async, [this] { tile_near_blocks(kNearQuadCols, near_quads); });
     NearTiling wide;
     tile_near_blocks(kNearTileCols, wide);
     near_tiles = std::move(wide.tiles);
     near_parts = wide.parts;
     near_slot = std::move(wide.slot);
     near_red_ptr = std::move(wide.red_ptr);
-    near_quads = NearTiling{};
-    if (near_entries <= kNearQuadEntries) tile_near_blocks(kNearQuadCols, near_quads);
 
     // Block rows: every stored block in both orientations.
     std::vector<int> leaf_of(n, -1);  // tree slot -> leaf node
@@ -986,6 +990,7 @@ void Plan::build_near_plan() {
         near_row_entries += static_cast<long long>(r.nrow) * r.ncol;
         near_rows.push_back(r);
     }
+    if (quads.valid()) quads.get();
 }
 
 // The stored blocks cut into tiles of at most cols columns.
