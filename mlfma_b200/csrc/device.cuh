@@ -61,10 +61,24 @@ struct DevStencilT {
     const R* coef_t;
 };
 
+// One (parent, child) pair of the anterpolation, with all its pointers.
+template <class R>
+struct DevL2LItem {
+    const typename Cx<R>::T* parent;  // the parent's local pattern
+    const typename Cx<R>::T* down;    // shift_down of the parent level, the child's octant
+    typename Cx<R>::T* child;         // the child's local pattern
+    const typename Cx<R>::T* up;      // shift_up of the child level, the child's octant
+};
+
 template <class R>
 struct DevTransT {
     DevStencilT<R> up_th, up_ph, dn_ph, dn_th;
     int plevel, npar;
+    int pth, pph, cth, cph;           // the parent's and the child's grid
+    const DevL2LItem<R>* l2l;         // in the order of the pair list
+    typename Cx<R>::T* const* par_a;  // [parent] its outgoing pattern
+    const typename Cx<R>::T* const* child_a;   // [child entry] its outgoing pattern
+    const typename Cx<R>::T* const* child_up;  //   and shift_up of its octant
     const int* par_box;
     const int* par_ilist;
     const int* child_ptr;

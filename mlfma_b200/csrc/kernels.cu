@@ -633,6 +633,31 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         d.child_ptr = upload(T.child_ptr);
         d.child_box = upload(T.child_box);
         d.child_oct = upload(T.child_oct);
+        d.pth = nth_[p];
+        d.pph = nph_[p];
+        d.cth = nth_[p + 1];
+        d.cph = nph_[p + 1];
+        const DevLevelT<R>& PD = F.lv[p];
+        const DevLevelT<R>& CD = F.lv[p + 1];
+        std::vector<C*> pa;
+        for (int b : T.par_box) pa.push_back(PD.A + static_cast<size_t>(b) * PD.ndir * 2);
+        std::vector<const C*> ca, cu;
+        for (size_t c = 0; c < T.child_box.size(); ++c) {
+            ca.push_back(CD.A + static_cast<size_t>(T.child_box[c]) * CD.ndir * 2);
+            cu.push_back(CD.shift_up + static_cast<size_t>(T.child_oct[c]) * CD.ndir);
+        }
+        std::vector<DevL2LItem<R>> items;
+        for (size_t q = 0; q < T.par_box.size(); ++q) {
+            if (ref_compat_ && !T.par_ilist[q]) continue;  // (the order of l2l_pairs_)
+            for (int c = T.child_ptr[q]; c < T.child_ptr[q + 1]; ++c)
+                items.push_back({PD.B + static_cast<size_t>(T.par_box[q]) * PD.ndir * 2,
+                                 PD.shift_down + static_cast<size_t>(T.child_oct[c]) * PD.ndir,
+                                 CD.B + static_cast<size_t>(T.child_box[c]) * CD.ndir * 2, cu[c]});
+        }
+        d.par_a = upload(pa);
+        d.child_a = upload(ca);
+        d.child_up = upload(cu);
+        d.l2l = upload(items);
     }
     if (std::is_same<R, double>::value) {
         F.pat = reinterpret_cast<C*>(const_cast<double2*>(pat64));
@@ -1173,11 +1198,11 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     const int rows = m2m_rows_[p];
     const dim3 grid(npar_[p], (nth_[p] + rows - 1) / rows);
     const DevTransT<R>& T = F.trans[p];
-    const size_t ssum = m2m_sum_smem(nth_[p + 1], nph_[p + 1], rows, sizeof(C));
+    const size_t ssum = m2m_sum_smem<R>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p]);
     if (!TR && m2m_pref_[p] && ssum + 1024 <= static_cast<size_t>(dev_smem_)) {
         const bool cs = m2m_pref_[p] == 2;
 #define MLFMA_M2M_SUM(WW) \
-    launch_k(pdl, cs ? k_m2m_sum<R, WW, true> : k_m2m_sum<R, WW, false>, grid, 256, ssum, s, F.lv_dev, T, rows)
+    launch_k(pdl, cs ? k_m2m_sum<R, WW, true> : k_m2m_sum<R, WW, false>, grid, 256, ssum, s, T, rows)
         switch (up_w_[p]) {
             case 2: MLFMA_M2M_SUM(2); break;
             case 4: MLFMA_M2M_SUM(4); break;
@@ -1250,7 +1275,7 @@ void DeviceOp::far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     const int g = n_l2l_pairs_[p];
     if (!g) return;
     const DevTransT<R>& T = F.trans[p];
-    const size_t sst = l2l_st_smem(nth_[p], nph_[p], nph_[p + 1], sizeof(C));
+    const size_t sst = l2l_st_smem<R>(nth_[p], nph_[p], nth_[p + 1], nph_[p + 1], dn_w_[p]);
     const size_t spipe = l2l_pipe_smem(nth_[p], nph_[p], nth_[p + 1], nph_[p + 1], sizeof(C));
     if (l2l_pref_[p] == 3 && spipe + 1024 <= static_cast<size_t>(dev_smem_)) {
         // persistent: as many blocks as fit on the SMs at once
@@ -1276,8 +1301,7 @@ void DeviceOp::far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     if (l2l_pref_[p] && l2l_pref_[p] != 3 && sst + 1024 <= static_cast<size_t>(dev_smem_)) {
         const bool cs = l2l_pref_[p] == 2;
 #define MLFMA_L2L_ST(WW)                                                                             \
-    launch_k(pdl, cs ? k_l2l_st<R, WW, TR, true> : k_l2l_st<R, WW, TR, false>, g, 256, sst, s, F.lv_dev, T, \
-             l2l_pairs_[p])
+    launch_k(pdl, cs ? k_l2l_st<R, WW, TR, true> : k_l2l_st<R, WW, TR, false>, g, 256, sst, s, T)
         switch (dn_w_[p]) {
             case 8: MLFMA_L2L_ST(8); break;
             case 12: MLFMA_L2L_ST(12); break;
@@ -2404,7 +2428,8 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
             for (int kind : {0, 1, 2})
                 for (int rows : {1, 2, 4, 8, 16, 32, 64}) {
                     if (rows > nth_[p] && rows != 1) continue;
-                    const size_t need = kind ? m2m_sum_smem(nth_[p + 1], nph_[p + 1], rows, csize) + 1024
+                    const size_t need = kind ? (precision_ == kFp64 ? m2m_sum_smem<double>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])
+                                                                    : m2m_sum_smem<float>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])) + 1024
                                              : static_cast<size_t>(8) * rows * nph_[p + 1] * 2 * csize;
                     if (need > static_cast<size_t>(dev_smem) || (!kind && rows > 16)) continue;
                     m2m_rows_[p] = rows;

@@ -99,8 +99,10 @@ k_s2m(const DevS2MItem<R>* __restrict__ items, const double2* __restrict__ x) {
 // shared memory; the sum is widened to complex double on output.
 //
 // HBM-bound (latency of the short rows: 3-5 KB a source).  Self-contained items
-// and the early loads: r = 2 sphere 45 -> 39 us, r = 8 sphere 597 -> 575 us
-// (4.8 TB/s); complex float 22 -> 18 us and 246 -> 183 us.  Blocks of 256
+// and the early loads: r = 2 sphere 45 -> 41 us, r = 8 sphere 597 -> 614 us
+// (4.5 TB/s); complex float 22 -> 18 us and 246 -> 183 us.  The four sums per
+// lane are a solve's: their order decides its last bits (two sums with twelve
+// loads in flight took 575 us on the r = 8 sphere).  Blocks of 256
 // threads left more warps idle at a leaf's last run of sources (FP64 598 us,
 // complex float 200 us on the r = 8 sphere).
 // CJ = false: plain patterns, y_m = sum_e R_m[e] b_B[e] -- the transpose of S2M,
@@ -744,32 +746,36 @@ k_l2l(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __restri
 // parent instead of one per child).  Block = (parent, tile of `rows` parent
 // theta rows); each child value is read from global memory once per block and
 // every stencil tap reads shared memory.
+//
+// Latency-bound: a block's life is its chain of dependent loads and its
+// barriers.  Grid sizes come with the launch, children as pointers, both
+// stencils are staged in shared memory while the children's values are on their
+// way, and every warp finds the band of child rows by itself.  With level
+// descriptors read by each block, shared atomics for the band and the stencils
+// from global memory: 181 against 173 us (complex float, sphere of radius 8
+// wavelengths, five transitions), 24 against 21.6 us (FP64, radius 2).
 template <class R, int W, bool CS>  // taps per row: 2 * interp_order (both passes); CS: column-stationary phi pass
 __global__ void __launch_bounds__(256)
-k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
+k_m2m_sum(DevTransT<R> T, int rows) {
     chain_wait();
     using C = typename Cx<R>::T;
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ int band[2];
     const int par = blockIdx.x;
-    const DevLevelT<R> P = lvs[T.plevel];
-    const DevLevelT<R> Cl = lvs[T.plevel + 1];
-    const int nph = P.nph, mph = Cl.nph, halfm = Cl.nph / 2;
+    const int nph = T.pph, mph = T.cph, halfm = T.cph / 2;
     const int r0 = blockIdx.y * rows;
-    const int nrow = min(P.nth, r0 + rows) - r0;
+    const int nrow = min(T.pth, r0 + rows) - r0;
     if (nrow <= 0) return;  // the whole block
-    if (threadIdx.x == 0) {
-        band[0] = Cl.nth;
-        band[1] = -1;
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < nrow * W; q += blockDim.x) {
+    const int c0 = T.child_ptr[par], nch = T.child_ptr[par + 1] - c0;
+    C* Ap = T.par_a[par] + static_cast<size_t>(r0) * nph * 2;
+    int lo = T.cth, hi = -1;
+    for (int q = threadIdx.x & 31; q < nrow * W; q += 32) {
         const int src = T.up_th.src[r0 * W + q];
-        atomicMin(&band[0], src);
-        atomicMax(&band[1], src);
+        lo = min(lo, src);
+        hi = max(hi, src);
     }
-    __syncthreads();
-    const int lo = band[0], nb = band[1] - lo + 1;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    const int nb = hi - lo + 1;
     // component planes (theta, phi), so that neighbouring threads read
     // neighbouring 8- or 16-byte words of shared memory
     const size_t nu = static_cast<size_t>(nb) * mph, nv = static_cast<size_t>(nrow) * mph;
@@ -777,34 +783,42 @@ k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
     C* U1 = U0 + nu;
     C* V0 = U1 + nu;                      // [nrow * mph]
     C* V1 = V0 + nv;
-    const int c0 = T.child_ptr[par], nch = T.child_ptr[par + 1] - c0;
+    R* th_cf = reinterpret_cast<R*>(V1 + nv);          // [nrow * W], then phi [W * nph] (tap-major)
+    R* ph_cf = th_cf + nrow * W;
+    int* th_src = reinterpret_cast<int*>(ph_cf + W * nph);  // row, reflected in bit 30
+    int* ph_src = th_src + nrow * W;
     for (int e = threadIdx.x; e < nb * mph; e += blockDim.x) {
         const int d = lo * mph + e;
         C u0 = zero<C>(), u1 = zero<C>();
 #pragma unroll 8
         for (int c = 0; c < nch; ++c) {
-            const C* Ac = Cl.A + static_cast<size_t>(T.child_box[c0 + c]) * Cl.ndir * 2;
-            const C ph = Cl.shift_up[static_cast<size_t>(T.child_oct[c0 + c]) * Cl.ndir + d];
+            const C ph = T.child_up[c0 + c][d];
             C x0, x1;
-            load_pair(Ac + 2 * d, x0, x1);
+            load_pair(T.child_a[c0 + c] + 2 * d, x0, x1);
             u0 = cfma(ph, x0, u0);
             u1 = cfma(ph, x1, u1);
         }
         U0[e] = u0;
         U1[e] = u1;
     }
+    for (int q = threadIdx.x; q < nrow * W; q += blockDim.x) {
+        th_cf[q] = T.up_th.coef[r0 * W + q];
+        th_src[q] = (T.up_th.src[r0 * W + q] - lo) | (T.up_th.refl[r0 * W + q] ? 1 << 30 : 0);
+    }
+    for (int q = threadIdx.x; q < W * nph; q += blockDim.x) {
+        ph_cf[q] = T.up_ph.coef_t[q];
+        ph_src[q] = T.up_ph.src_t[q];
+    }
     __syncthreads();
     for (int it = threadIdx.x; it < nrow * mph; it += blockDim.x) {
         const int jr = it / mph, iph = it - jr * mph;
-        const int jth = r0 + jr;
+        const int iref = iph < halfm ? iph + halfm : iph - halfm;
         C v0 = zero<C>(), v1 = zero<C>();
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            const int q = jth * W + k;
-            const bool rf = T.up_th.refl[q];
-            const int sp = rf ? (iph < halfm ? iph + halfm : iph - halfm) : iph;
-            const R cf = T.up_th.coef[q];
-            const int e = (T.up_th.src[q] - lo) * mph + sp;
+            const int q = th_src[jr * W + k];
+            const R cf = th_cf[jr * W + k];
+            const int e = (q & ~(1 << 30)) * mph + (q >> 30 ? iref : iph);
             v0 = crfma(cf, U0[e], v0);
             v1 = crfma(cf, U1[e], v1);
         }
@@ -812,7 +826,6 @@ k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
         V1[it] = v1;
     }
     __syncthreads();
-    C* Ap = P.A + (static_cast<size_t>(T.par_box[par]) * P.ndir + static_cast<size_t>(r0) * nph) * 2;
     if (!CS) {  // one output per thread, stencil read per tap (tap-major)
         for (int o = threadIdx.x; o < nrow * nph; o += blockDim.x) {
             const int jr = o / nph, jph = o - jr * nph;
@@ -822,8 +835,8 @@ k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
 #pragma unroll
             for (int k = 0; k < W; ++k) {
                 const int q = k * nph + jph;
-                const int s = T.up_ph.src_t[q];
-                const R cf = T.up_ph.coef_t[q];
+                const int s = ph_src[q];
+                const R cf = ph_cf[q];
                 a0 = crfma(cf, row0[s], a0);
                 a1 = crfma(cf, row1[s], a1);
             }
@@ -840,8 +853,8 @@ k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
         R ck[W];
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            sk[k] = T.up_ph.src_t[k * nph + jph];
-            ck[k] = T.up_ph.coef_t[k * nph + jph];
+            sk[k] = ph_src[k * nph + jph];
+            ck[k] = ph_cf[k * nph + jph];
         }
         for (int jr = g; jr < nrow; jr += ng) {
             const C* row0 = V0 + static_cast<size_t>(jr) * mph;
@@ -860,42 +873,58 @@ k_m2m_sum(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, int rows) {
 
 // Shared memory of k_m2m_sum for a tile of `rows` parent rows (bound: every
 // child row in the band).
-inline size_t m2m_sum_smem(int child_nth, int child_nph, int rows, size_t csize) {
-    return static_cast<size_t>(child_nth + rows) * child_nph * 2 * csize;
+template <class R>
+size_t m2m_sum_smem(int child_nth, int parent_nph, int child_nph, int rows, int w) {
+    return static_cast<size_t>(child_nth + rows) * child_nph * 2 * sizeof(typename Cx<R>::T) +
+           static_cast<size_t>(rows + parent_nph) * w * (sizeof(R) + sizeof(int));
 }
 
 // L2L (and, POST, the transposed M2M) with the parent's local pattern, shifted
 // to the child's octant, staged in shared memory once per block: the same
 // arithmetic in the same order as k_l2l, every phi tap then reading shared
 // memory instead of global memory.  One block per (parent, child) pair.
+//
+// Latency-bound as k_m2m_sum: one load finds a pair's pointers, the stencils are
+// staged beside the parent's values, and the child's pattern is requested before
+// the last pass.  Without these (level descriptor, pair, box and octant read one
+// after the other): 337 against 288 us (complex float, sphere of radius 8
+// wavelengths, five transitions), 38 against 31.7 us (FP64, radius 2).
 template <class R, int W, bool POST, bool CS>  // both transposed stencils padded to W taps per row
 __global__ void __launch_bounds__(256)
-k_l2l_st(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __restrict__ pairs) {
+k_l2l_st(DevTransT<R> T) {
     chain_wait();
     using C = typename Cx<R>::T;
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int2 pc = pairs[blockIdx.x];  // parent index, child entry
-    const DevLevelT<R> P = lvs[T.plevel];
-    const DevLevelT<R> Cl = lvs[T.plevel + 1];
-    const int pth = P.nth, pph = P.nph, cth = Cl.nth, cph = Cl.nph, halfc = Cl.nph / 2;
+    const DevL2LItem<R> it = T.l2l[blockIdx.x];
+    const int pth = T.pth, pph = T.pph, cth = T.cth, cph = T.cph, halfc = T.cph / 2;
     // component planes (theta, phi): neighbouring threads read neighbouring words
     const size_t np = static_cast<size_t>(pth) * pph, nq = static_cast<size_t>(pth) * cph;
     C* SB0 = reinterpret_cast<C*>(smraw);  // [pth * pph]
     C* SB1 = SB0 + np;
     C* S10 = SB1 + np;                     // [pth * cph]
     C* S11 = S10 + nq;
-    const C* Bp = P.B + static_cast<size_t>(T.par_box[pc.x]) * P.ndir * 2;
-    const C* sh = P.shift_down + static_cast<size_t>(T.child_oct[pc.y]) * P.ndir;
+    R* ph_cf = reinterpret_cast<R*>(S11 + nq);              // [W * cph] (tap-major), then theta [cth * W]
+    R* th_cf = ph_cf + W * cph;
+    int* ph_src = reinterpret_cast<int*>(th_cf + cth * W);
+    int* th_src = ph_src + W * cph;                         // row, reflected in bit 30
     for (int d = threadIdx.x; d < pth * pph; d += blockDim.x) {
         C b0, b1;
-        load_pair(Bp + 2 * d, b0, b1);
+        load_pair(it.parent + 2 * d, b0, b1);
         if (!POST) {
-            const C ph = sh[d];
+            const C ph = it.down[d];
             b0 = cmul(ph, b0);
             b1 = cmul(ph, b1);
         }
         SB0[d] = b0;
         SB1[d] = b1;
+    }
+    for (int q = threadIdx.x; q < W * cph; q += blockDim.x) {
+        ph_cf[q] = T.dn_ph.coef_t[q];
+        ph_src[q] = T.dn_ph.src_t[q];
+    }
+    for (int q = threadIdx.x; q < cth * W; q += blockDim.x) {
+        th_cf[q] = T.dn_th.coef[q];
+        th_src[q] = T.dn_th.src[q] | (T.dn_th.refl[q] ? 1 << 30 : 0);
     }
     __syncthreads();
     if (!CS) {  // one output per thread, stencil read per tap (tap-major)
@@ -906,9 +935,8 @@ k_l2l_st(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __res
             C v0 = zero<C>(), v1 = zero<C>();
 #pragma unroll
             for (int k = 0; k < W; ++k) {
-                const int q = k * cph + jph;
-                const int d = T.dn_ph.src_t[q];
-                const R cf = T.dn_ph.coef_t[q];
+                const int d = ph_src[k * cph + jph];
+                const R cf = ph_cf[k * cph + jph];
                 v0 = crfma(cf, row0[d], v0);
                 v1 = crfma(cf, row1[d], v1);
             }
@@ -925,8 +953,8 @@ k_l2l_st(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __res
         R ck[W];
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            sk[k] = T.dn_ph.src_t[k * cph + jph];
-            ck[k] = T.dn_ph.coef_t[k * cph + jph];
+            sk[k] = ph_src[k * cph + jph];
+            ck[k] = ph_cf[k * cph + jph];
         }
         for (int ith = g; ith < pth; ith += ng) {
             const C* row0 = SB0 + static_cast<size_t>(ith) * pph;
@@ -942,28 +970,26 @@ k_l2l_st(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __res
         }
     }
     __syncthreads();
-    C* Bc = Cl.B + static_cast<size_t>(T.child_box[pc.y]) * Cl.ndir * 2;
     for (int e = threadIdx.x; e < cth * cph; e += blockDim.x) {
         const int jth = e / cph, jph = e - jth * cph;
+        const int jref = jph < halfc ? jph + halfc : jph - halfc;
         C c0, c1;  // the child's local pattern, in flight during the taps
-        load_pair(Bc + 2 * e, c0, c1);
+        load_pair(it.child + 2 * e, c0, c1);
         C v0 = zero<C>(), v1 = zero<C>();
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            const int q = jth * W + k;
-            const bool rf = T.dn_th.refl[q];
-            const int sp = rf ? (jph < halfc ? jph + halfc : jph - halfc) : jph;
-            const R cf = T.dn_th.coef[q];
-            const size_t at = static_cast<size_t>(T.dn_th.src[q]) * cph + sp;
+            const int q = th_src[jth * W + k];
+            const R cf = th_cf[jth * W + k];
+            const int at = (q & ~(1 << 30)) * cph + (q >> 30 ? jref : jph);
             v0 = crfma(cf, S10[at], v0);
             v1 = crfma(cf, S11[at], v1);
         }
         if (POST) {
-            const C ph = Cl.shift_up[static_cast<size_t>(T.child_oct[pc.y]) * Cl.ndir + e];
+            const C ph = it.up[e];
             v0 = cmul(ph, v0);
             v1 = cmul(ph, v1);
         }
-        store_pair(Bc + 2 * e, cadd(c0, v0), cadd(c1, v1));
+        store_pair(it.child + 2 * e, cadd(c0, v0), cadd(c1, v1));
     }
 }
 
@@ -1087,8 +1113,10 @@ inline size_t l2l_pipe_smem(int pth, int pph, int cth, int cph, size_t csize) {
     return (2 * per_buf + 2 * np + 2 * static_cast<size_t>(pth) * cph) * csize;
 }
 
-inline size_t l2l_st_smem(int parent_nth, int parent_nph, int child_nph, size_t csize) {
-    return static_cast<size_t>(parent_nth) * (parent_nph + child_nph) * 2 * csize;
+template <class R>
+size_t l2l_st_smem(int parent_nth, int parent_nph, int child_nth, int child_nph, int w) {
+    return static_cast<size_t>(parent_nth) * (parent_nph + child_nph) * 2 * sizeof(typename Cx<R>::T) +
+           static_cast<size_t>(child_nph + child_nth) * w * (sizeof(R) + sizeof(int));
 }
 
 // Complex double -> far-field type (patterns, tables at setup).
