@@ -182,8 +182,10 @@ int mlfma_get_stats(mlfma_handle h, mlfma_stats* st);
 int mlfma_rhs(mlfma_handle h, double* b);
 
 /* y = A x (accumulate = 0) or y += A x (accumulate = 1), host buffers
- * (Solver::evalRvec, src/solver.cpp:41-57: rvec += A lvec).  Copies in and
- * out through the handle's stream. */
+ * (Solver::evalRvec, src/solver.cpp:41-57: rvec += A lvec).  Complete on
+ * return.  Ordinary memory of up to 262,144 unknowns goes through the handle's
+ * page-locked buffer (32 bytes per unknown, allocated at setup), the rest
+ * through the driver's copies, on the handle's stream. */
 int mlfma_matvec(mlfma_handle h, const double* x, double* y, int accumulate);
 
 /* Same on device buffers (cudaStream_t passed as void*, NULL = handle's stream).

@@ -28,13 +28,16 @@ struct mlfma_op_s {
     double2* d_ym = nullptr;
     double2* d_x = nullptr;  // staging for host-buffer calls
     double2* d_y = nullptr;
+    double2* h_pin = nullptr;   // page-locked, mapped: x and y of a host-buffer product (host_product)
+    double2* d_pin = nullptr;   // its device address
     void* d_stage = nullptr;  // small per-call inputs and outputs (directions, rows, far fields); grows only
     size_t stage_bytes = 0;
     mlfma_op_s* inner = nullptr;        // operator of the flexible solve's inner iterations
     std::vector<mlfma_op_s*> outers;    // operators that use this one as their inner operator
     ~mlfma_op_s() {
-        if (d_x || d_y || d_xm || d_ym || d_stage) {
+        if (d_x || d_y || d_xm || d_ym || d_stage || h_pin) {
             cudaSetDevice(device);
+            if (h_pin) cudaFreeHost(h_pin);
             if (d_x) cudaFree(d_x);
             if (d_y) cudaFree(d_y);
             if (d_xm) cudaFree(d_xm);
@@ -103,6 +106,57 @@ mlfma::PlaneWave to_pw(const mlfma_planewave* p) {
 }
 
 bool ready(mlfma_handle h) { return h && h->dev; }
+
+// Largest vector (unknowns) that a product on ordinary host memory stages
+// itself.  The driver copies such memory through its own page-locked buffers, in
+// a blocking call on either side of the product; here the vector is copied into
+// the handle's page-locked buffer, and the gathering and finishing kernels read
+// and write it over the bus (as mlfma_matvec_mapped).  FP64 product, driver's
+// copies -> staged: 80 -> 53 us (1,920 unknowns), 126 -> 98 us (7,680, adjoint),
+// 335 -> 280 us (30,720), 1,175 -> 1,112 us (122,880); at 491,520 the two are
+// within 4 % and page-locking 16 MB would be paid for at setup.
+constexpr int kPinnedVector = 1 << 18;
+
+bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// y (+)= A x or A^H x on host buffers, complete on return.  Page-locked, managed
+// and device addresses keep the driver's copies (and its errors).
+int host_product(mlfma_handle h, const double* x, double* y, bool accumulate, bool adj) {
+    if (!h || !x || !y) return fail(MLFMA_ERR_ARG, "null argument");
+    if (!ready(h)) return fail(MLFMA_ERR_STATE, "mlfma_setup has not run");
+    const int n = h->plan.n;
+    const size_t bytes = sizeof(double2) * n;
+    cudaStream_t s = h->dev->stream();
+    if (cudaSetDevice(h->device) != cudaSuccess) return fail(MLFMA_ERR_CUDA, "cudaSetDevice failed");
+    if (h->d_pin && pageable(x) && pageable(y)) {
+        std::memcpy(h->h_pin, x, bytes);
+        if (accumulate) std::memcpy(h->h_pin + n, y, bytes);
+        std::string e = h->dev->matvec_mapped(h->d_pin, h->d_pin + n, accumulate, s, adj);
+        if (!e.empty()) return from_msg(e);
+        const cudaError_t ce = cudaStreamSynchronize(s);
+        if (ce != cudaSuccess) return fail(MLFMA_ERR_CUDA, cudaGetErrorString(ce));
+        std::memcpy(y, h->h_pin + n, bytes);
+        return MLFMA_OK;
+    }
+    if (cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
+        return fail(MLFMA_ERR_CUDA, "copy of x failed");
+    if (accumulate && cudaMemcpyAsync(h->d_y, y, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
+        return fail(MLFMA_ERR_CUDA, "copy of y failed");
+    std::string e = h->dev->matvec_device(h->d_x, h->d_y, accumulate, s, -1, adj);
+    if (!e.empty()) return from_msg(e);
+    if (cudaMemcpyAsync(y, h->d_y, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+        return fail(MLFMA_ERR_CUDA, "copy of y failed");
+    const cudaError_t ce = cudaStreamSynchronize(s);
+    if (ce != cudaSuccess) return fail(MLFMA_ERR_CUDA, cudaGetErrorString(ce));
+    return MLFMA_OK;
+}
 
 }  // namespace
 
@@ -183,6 +237,15 @@ int mlfma_setup(mlfma_handle h) {
         if (cudaMalloc(&h->d_x, sizeof(double2) * h->plan.n) != cudaSuccess ||
             cudaMalloc(&h->d_y, sizeof(double2) * h->plan.n) != cudaSuccess)
             return fail(MLFMA_ERR_CUDA, "cudaMalloc failed");
+        if (h->plan.n <= kPinnedVector) {  // without it products copy through the driver
+            void* p = nullptr;
+            void* d = nullptr;
+            if (cudaHostAlloc(&p, 2 * sizeof(double2) * h->plan.n, cudaHostAllocMapped) == cudaSuccess) {
+                h->h_pin = static_cast<double2*>(p);
+                if (cudaHostGetDevicePointer(&d, p, 0) == cudaSuccess) h->d_pin = static_cast<double2*>(d);
+            }
+            if (!h->d_pin) cudaGetLastError();
+        }
         // The fixed workspace of mlfma_gmres_noalloc is created on this device
         // now (first use of its module), not inside a solve.
         e = mlfma::noalloc_workspace_prepare();
@@ -226,22 +289,9 @@ int mlfma_rhs(mlfma_handle h, double* b) {
 }
 
 int mlfma_matvec(mlfma_handle h, const double* x, double* y, int accumulate) {
-    if (!h || !x || !y) return fail(MLFMA_ERR_ARG, "null argument");
-    if (!ready(h)) return fail(MLFMA_ERR_STATE, "mlfma_setup has not run");
-    const size_t bytes = sizeof(double2) * h->plan.n;
-    cudaStream_t s = h->dev->stream();
-    if (cudaSetDevice(h->device) != cudaSuccess) return fail(MLFMA_ERR_CUDA, "cudaSetDevice failed");
-    if (cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of x failed");
-    if (accumulate && cudaMemcpyAsync(h->d_y, y, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of y failed");
-    std::string e = h->dev->matvec_device(h->d_x, h->d_y, accumulate != 0, s);
-    if (!e.empty()) return fail(MLFMA_ERR_CUDA, e);
-    if (cudaMemcpyAsync(y, h->d_y, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of y failed");
-    const cudaError_t ce = cudaStreamSynchronize(s);
-    if (ce != cudaSuccess) return fail(MLFMA_ERR_CUDA, cudaGetErrorString(ce));
-    e = h->dev->device_error();
+    const int rc = host_product(h, x, y, accumulate != 0, false);
+    if (rc != MLFMA_OK) return rc;
+    const std::string e = h->dev->device_error();
     if (!e.empty()) return fail(MLFMA_ERR_CUDA, e);
     return MLFMA_OK;
 }
@@ -602,22 +652,7 @@ int mlfma_set_loads(mlfma_handle h, const double* z) {
 }
 
 int mlfma_matvec_adjoint(mlfma_handle h, const double* x, double* y, int accumulate) {
-    if (!h || !x || !y) return fail(MLFMA_ERR_ARG, "null argument");
-    if (!ready(h)) return fail(MLFMA_ERR_STATE, "mlfma_setup has not run");
-    const size_t bytes = sizeof(double2) * h->plan.n;
-    cudaStream_t s = h->dev->stream();
-    if (cudaSetDevice(h->device) != cudaSuccess) return fail(MLFMA_ERR_CUDA, "cudaSetDevice failed");
-    if (cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of x failed");
-    if (accumulate && cudaMemcpyAsync(h->d_y, y, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of y failed");
-    std::string e = h->dev->matvec_device(h->d_x, h->d_y, accumulate != 0, s, -1, true);
-    if (!e.empty()) return from_msg(e);
-    if (cudaMemcpyAsync(y, h->d_y, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-        return fail(MLFMA_ERR_CUDA, "copy of y failed");
-    const cudaError_t ce = cudaStreamSynchronize(s);
-    if (ce != cudaSuccess) return fail(MLFMA_ERR_CUDA, cudaGetErrorString(ce));
-    return MLFMA_OK;
+    return host_product(h, x, y, accumulate != 0, true);
 }
 
 static mlfma::SolveOpts to_opts(const mlfma_solver_opts* opts) {

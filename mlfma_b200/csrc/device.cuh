@@ -287,7 +287,7 @@ public:
     // mapped; device-side addresses of them): the gather kernel reads x and
     // the finishing kernel writes y in caller order straight over the bus
     // (coalesced), no separate copies.
-    std::string matvec_mapped(const double2* x, double2* y, bool accumulate, cudaStream_t stream);
+    std::string matvec_mapped(const double2* x, double2* y, bool accumulate, cudaStream_t stream, bool adj = false);
 
     // Non-empty when a kernel of this operator gave up a bounded wait (its
     // results since then are not valid); read after the stream is synchronised.

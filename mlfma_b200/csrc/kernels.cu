@@ -99,20 +99,25 @@ __global__ void k_finish(const double2* __restrict__ yfar, const double2* __rest
 // The boundary kernels of a product on mapped host buffers, indexed by the
 // caller's order so that every warp reads x and writes y in one contiguous
 // run across the bus: xt[tpos[c]] = x[c]; y[c] (+)= ck (yfar + ynear)[tpos[c]]
-// + loads xt (the same value k_finish forms).
+// + loads xt, both conjugated when cj (the same values k_gather and k_finish form).
 __global__ void k_gather_caller(const double2* __restrict__ x, const int* __restrict__ tpos,
-                                double2* __restrict__ xt, int n) {
+                                double2* __restrict__ xt, int n, int cj) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < n) xt[tpos[c]] = x[c];
+    if (c >= n) return;
+    double2 v = x[c];
+    if (cj) v.y = -v.y;
+    xt[tpos[c]] = v;
 }
 __global__ void k_finish_caller(const double2* __restrict__ yfar, const double2* __restrict__ ynear,
                                 const int* __restrict__ tpos, double2* __restrict__ y, int n, double2 ck,
-                                int accumulate, const double2* __restrict__ xt, const double2* __restrict__ loads) {
+                                int accumulate, const double2* __restrict__ xt, const double2* __restrict__ loads,
+                                int cj) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
     const int t = tpos[c];
     double2 v = cmul(ck, cadd(yfar[t], ynear[t]));
     if (loads) v = cfma(loads[t], xt[t], v);
+    if (cj) v.y = -v.y;
     y[c] = accumulate ? cadd(y[c], v) : v;
 }
 
@@ -1557,16 +1562,17 @@ std::string DeviceOp::matvec_device(const double2* x, double2* y, bool accumulat
     return {};
 }
 
-std::string DeviceOp::matvec_mapped(const double2* x, double2* y, bool accumulate, cudaStream_t stream) {
+std::string DeviceOp::matvec_mapped(const double2* x, double2* y, bool accumulate, cudaStream_t stream, bool adj) {
     if (!ready_) return "operator not set up";
+    if (adj && ref_compat_) return "arg:the adjoint needs ref_compat = 0 (the reference's rule keeps state between products)";
     cudaStream_t s = stream ? stream : stream_;
     MLFMA_CK(cudaSetDevice(device_));
-    std::string e = ensure_graph(precision_, false, false);
+    std::string e = ensure_graph(precision_, adj, false);
     if (!e.empty()) return e;
-    k_gather_caller<<<blocks_for(n_, 256), 256, 0, s>>>(x, tpos_, xt_, n_);
-    launch_core(s, precision_, false, false);
+    k_gather_caller<<<blocks_for(n_, 256), 256, 0, s>>>(x, tpos_, xt_, n_, adj ? 1 : 0);
+    launch_core(s, precision_, adj, false);
     k_finish_caller<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, tpos_, y, n_, ck_, accumulate ? 1 : 0, xt_,
-                                                        has_loads_ ? loads_ : nullptr);
+                                                        has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
     MLFMA_CK(cudaGetLastError());
     return {};
 }
