@@ -1091,8 +1091,7 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
                     n_near_quads_ = static_cast<int>(quads.size() / 4);
                     near_quads_ = upload(quads);
                 }
-                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_) + kNearPad);
-                MLFMA_CK(cudaMemsetAsync(near_bz_ + near_block_entries_, 0, sizeof(double2) * kNearPad, stream_));
+                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_));
                 near_part_ = alloc<double2>(parts);
                 near_red_ptr_ = upload(plan.near_red_ptr);
                 near_slot_ = upload(plan.near_slot);

@@ -300,12 +300,10 @@ __device__ __forceinline__ double2 halve(double2 a, double2 b, bool hi, int mask
 // column count overran the instruction cache, 85 us; entries by cp.async or bulk
 // copies in shared-memory rings, with the fewer warps those leave, 75 and 55 us.
 //
-// A rectangular row is read to the end of the last column group it starts in:
-// past its end lies the next row or tile (kNearPad zeros after the last), which
-// meets an x of zero and a column sum that is not written.  A self tile's
-// diagonal counts once, in its row.
+// Only entries of a lane's own row are read, and a self block's row takes no x
+// from beyond its end, so an entry or an x that is not finite spoils the sums it
+// belongs to and no other.  A self tile's diagonal counts once, in its row.
 constexpr int kNdThreads = 128;
-constexpr int kNearPad = 8;
 
 template <bool SELF>
 __device__ __forceinline__ void near_quad(const DevNearTile& T, const double2* __restrict__ Z,
@@ -352,7 +350,7 @@ __device__ __forceinline__ void near_quad(const DevNearTile& T, const double2* _
 #pragma unroll
             for (int j = 0; j < G; ++j) {
                 z[i][j] = z0();
-                if (j < gmax && (SELF ? lc + 8 * j : 8 * j) < len) z[i][j] = __ldcs(zr + 8 * j);
+                if (j < gmax && lc + 8 * j < len) z[i][j] = __ldcs(zr + 8 * j);
             }
         }
         const int rslot = (lc & 1) == 0 && rb + ro < T.ni ? sl[rb + ro] : -1;
@@ -362,7 +360,7 @@ __device__ __forceinline__ void near_quad(const DevNearTile& T, const double2* _
 #pragma unroll
             for (int j = 0; j < G; ++j) {
                 if (j >= gmax) break;
-                p[i] = cfma(z[i][j], xc[j], p[i]);
+                if (!SELF || rb + i + T.kind > lc + 8 * j + dcol + 1) p[i] = cfma(z[i][j], xc[j], p[i]);
                 if (!SELF || rb + i > lc + 8 * j + dcol) ca[j] = cfma(z[i][j], xv[i], ca[j]);
             }
         }

@@ -36,3 +36,31 @@ def test_two_leaves(cuda_device, na, nb):
     r = np.random.default_rng(na + 100 * nb)
     a, b = r.uniform(0.05, 0.45, (na, 3)), -r.uniform(0.05, 0.45, (nb, 3))
     check(np.concatenate([a, b]), 1, max(na, nb))
+
+
+@pytest.mark.parametrize("at", [0, 20, 39])
+def test_not_finite_stays_where_it_belongs(cuda_device, at):
+    # one x of NaN and one pair of sources in one place (an entry that is not
+    # finite): exactly the sums that contain them are not finite
+    r = np.random.default_rng(4)
+    pos = r.uniform(-1, 1, (40, 3))
+    d = inputs.Dipoles(pos=pos, mom=np.tile([1.0, 2.0, -0.5], (40, 1)))
+    op = MLFMA.dipoles(d, PW, max_node_srcs=64, self_terms=0, ref_compat=0).setup()
+    x = r.standard_normal(op.n) + 1j * r.standard_normal(op.n)
+    x[at] = np.nan
+    masks = []
+    for kind in (2, 0):
+        op.set_near_kernel(kind)
+        masks.append(np.isfinite(op.matvec(x)))
+    assert masks[0][at] and masks[0].sum() == 1  # (no self term: every other sum has it)
+    assert np.array_equal(masks[0], masks[1])
+    op.close()
+    pos[at] = pos[(at + 7) % 40]
+    op = MLFMA.dipoles(inputs.Dipoles(pos=pos, mom=d.mom), PW, max_node_srcs=64, self_terms=0, ref_compat=0).setup()
+    x[at] = 1.0
+    masks = []
+    for kind in (2, 0):
+        op.set_near_kernel(kind)
+        masks.append(np.isfinite(op.matvec(x)))
+    assert np.array_equal(masks[0], masks[1])
+    op.close()
