@@ -349,7 +349,8 @@ typedef struct {
     float product_ms_after;
     int near_blocks_per_sm;    /* one-vector near field: persistent blocks per SM (it runs beside the far field) */
     int interp_path;           /* interpolation/anterpolation kernels chosen (see mlfma_set_interp_path) */
-    int schedule;              /* one-vector product: bit 0 translation lists staged in shared memory,
+    int schedule;              /* one-vector product: bit 0 translation lists staged in shared memory
+                                  (complex double: sibling boxes translated together),
                                   bit 1 near field started after aggregation, bit 2 two side streams
                                   for the finer levels' translations, bit 3 the far-field chain's
                                   kernels launched as programmatic dependent launches (each kernel's
@@ -362,8 +363,8 @@ typedef struct {
                                   column-stationary phi passes, bit 24 + p = the persistent prefetching
                                   kernel */
     int near_kernel;           /* one-vector near field: 0 one tile per thread block (row and column
-                                  threads), 1 one tile per warp from shared memory, 2 one tile per
-                                  warp from global memory (see mlfma_set_near_kernel) */
+                                  threads), 2 four tiles per warp from global memory (see
+                                  mlfma_set_near_kernel) */
 } mlfma_tuning;
 
 /* Autotuner: times the candidate launch shapes of the stages on this operator
@@ -403,17 +404,19 @@ int mlfma_get_interp_path(mlfma_handle h, int* mode);
 int mlfma_set_staged_interp(mlfma_handle h, int mode);
 /* Near-field kernel of the one-vector product (Leaf::evalPairSols,
  * evalNearNonNborSols, evalSelfSols, src/fmm/leaf.cpp:318-383; each stored block
- * applied as Z and Z^T, tiles streamed by bulk copies): kind 0, one tile per
- * thread block (row threads and column threads; the default); kind 1, one
- * tile per warp, each entry read from shared memory once and the row sums
- * formed by a warp reduce-scatter; kind 2, one tile per warp with the entries
- * loaded straight from global memory into registers (no shared-memory stage).
- * Same partial sums, other rounding order; mlfma_autotune tries all three. */
+ * applied as Z and Z^T): kind 0, one tile of up to 64 columns per thread block,
+ * streamed by bulk copies (row threads and column threads); kinds 1 and 2, four
+ * tiles of up to 32 columns per warp, the entries loaded straight from global
+ * memory into registers.  The latter is the default up to 50,331,648 stored
+ * entries; above, only kind 0 exists and every kind means it.  A mixed
+ * operator's solves always use kind 0 (their last bits follow its order).  Same
+ * products, other rounding order; mlfma_autotune tries both. */
 int mlfma_set_near_kernel(mlfma_handle h, int kind);
 
 /* The one-vector product's schedule, as mlfma_tuning.schedule reports it (no
  * counterpart in the reference, which runs the stages one after another on
- * one thread): bit 0 translation lists staged in shared memory, bit 1 near
+ * one thread): bit 0 translation lists staged in shared memory (an FP64
+ * operator's larger levels: sibling boxes translated together), bit 1 near
  * field started after aggregation, bit 2 two side streams for the finer
  * levels' translations, bit 3 the far-field chain's kernels launched as
  * programmatic dependent launches.  Results are unchanged up to rounding

@@ -280,7 +280,7 @@ class MLFMA:
         check(lib().mlfma_set_schedule(self._h, int(schedule)))
 
     def set_near_kernel(self, kind: int) -> None:
-        """0: one near-field tile per thread block; 1: one per warp (mlfma_set_near_kernel)."""
+        """0: one near-field tile per thread block; 1 or 2: four per warp (mlfma_set_near_kernel)."""
         check(lib().mlfma_set_near_kernel(self._h, int(kind)))
 
     def set_inner_operator(self, inner: "MLFMA | None") -> None:

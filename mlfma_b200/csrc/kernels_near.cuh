@@ -292,7 +292,7 @@ __device__ __forceinline__ double2 halve(double2 a, double2 b, bool hi, int mask
 // rectangular or all self, by column groups and rows), so that a warp's tiles
 // end together.
 //
-// Bound by memory latency at 12 warps per SM (ncu, 7.8M entries: 50 us cold, 36 %
+// Bound by memory latency at 12 warps per SM (ncu, 7.8M entries: 46 us cold, 37 %
 // of DRAM, issue 27 %); what it gains on k_near_sym, as fast alone (43 us),
 // is what it leaves to the far-field chain beside it: no shared memory, half the
 // issue slots.  Measured on the way: one tile per warp (lanes 4 x 8 over the
