@@ -425,6 +425,7 @@ private:
     void far_l2l_tc(int p, int nr, cudaStream_t s);
     void drop_graphs();
     static int m2m_rows(int nth, int nph);
+    int m2m_sum_rows(int nth, int npar) const;
 
     int device_ = 0;
     int n_ = 0;
@@ -461,7 +462,8 @@ private:
     // -> 184 us, r = 4 sphere 751 -> 737 us, 50,000 dipoles 604 -> 599 us)
     int m2l_streams_ = 2;
     bool chain_pdl_ = false;              // far-field chain kernels as programmatic dependent launches
-    std::vector<int> m2m_rows_;           // one-vector M2M parent rows per block, per transition
+    std::vector<int> m2m_rows_;           // one-vector M2M parent rows per block, per transition (k_m2m)
+    std::vector<int> m2m_sum_rows_;       //   and of k_m2m_sum
     std::vector<int> m2m_pref_, l2l_pref_;  // per transition: 1 = staged kernels (k_m2m_sum, k_l2l_st) where they fit
     int dev_smem_ = 0;                    // opt-in shared memory per block
     int near_kernel_ = 0;                 // one-vector near field: 0 k_near_sym, 1 or 2 k_near_direct (where there are quads)

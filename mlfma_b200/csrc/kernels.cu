@@ -217,6 +217,18 @@ int DeviceOp::m2m_rows(int nth, int nph) {
     return std::max(1, std::min(nth, 128 / std::max(nph, 1)));
 }
 
+// Parent rows per block of k_m2m_sum.  A block sums the children on the band of
+// child rows its rows' stencils read, about rows / 2 + 6 of them, so few rows
+// repeat that work; up to 16, as long as there are two blocks per SM.  One
+// parent output per thread, as k_m2m has it (one to four rows): r = 8 sphere, five
+// transitions, complex float 173 us, this 105 us; FP64 306 us, this 173 us.
+int DeviceOp::m2m_sum_rows(int nth, int npar) const {
+    int rows = 1;
+    while (rows < 16 && 2 * rows <= nth && static_cast<long long>(npar) * ((nth + 2 * rows - 1) / (2 * rows)) >= 2 * sms_)
+        rows *= 2;
+    return rows;
+}
+
 // One-vector M2L work items (level, box, first direction, count) for a
 // direction chunk of at most max_chunk, written to the device array; items of
 // each level are contiguous (m2l_first_, m2l_count_).
@@ -902,6 +914,7 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
         // ---- transitions: L2L pairs and stencil widths
         l2l_pairs_.assign(std::max(lmax_, 0) + 1, nullptr);
         m2m_rows_.assign(std::max(lmax_, 0) + 1, 1);
+        m2m_sum_rows_.assign(std::max(lmax_, 0) + 1, 1);
         m2m_pref_.assign(std::max(lmax_, 0) + 1, 0);
         l2l_pref_.assign(std::max(lmax_, 0) + 1, 0);
         MLFMA_CK(cudaDeviceGetAttribute(&dev_smem_, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
@@ -931,6 +944,7 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
             m2m_pref_[p] = 1;
             l2l_pref_[p] = 1;
             npar_[p] = static_cast<int>(T.par_box.size());
+            m2m_sum_rows_[p] = m2m_sum_rows(nth_[p], npar_[p]);
             std::vector<int2> pairs;
             for (int q = 0; q < npar_[p]; ++q) {
                 if (ref_compat_ && !T.par_ilist[q]) continue;  // stem.cpp:115
@@ -1199,9 +1213,9 @@ template <class R, bool TR>
 void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     using C = typename Cx<R>::T;
     if (npar_[p] == 0) return;
-    const int rows = m2m_rows_[p];
-    const dim3 grid(npar_[p], (nth_[p] + rows - 1) / rows);
     const DevTransT<R>& T = F.trans[p];
+    int rows = m2m_sum_rows_[p];
+    dim3 grid(npar_[p], (nth_[p] + rows - 1) / rows);
     const size_t ssum = m2m_sum_smem<R>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p]);
     if (!TR && m2m_pref_[p] && ssum + 1024 <= static_cast<size_t>(dev_smem_)) {
         const bool cs = m2m_pref_[p] == 2;
@@ -1217,6 +1231,8 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
 #undef MLFMA_M2M_SUM
         return;
     }
+    rows = m2m_rows_[p];
+    grid.y = (nth_[p] + rows - 1) / rows;
     const size_t smem = static_cast<size_t>(8) * rows * nph_[p + 1] * 2 * sizeof(C);
     switch (up_w_[p]) {
         case 2: launch_k(pdl, k_m2m<R, 2, TR>, grid, 128, smem, s, F.lv_dev, T, rows); break;
@@ -2429,7 +2445,8 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
         for (int p = lmin_; p < lmax_; ++p) {
             if (!npar_[p]) continue;
             float bt = 1e30f;
-            int brows = m2m_rows_[p], bkind = m2m_pref_[p];
+            const int rows0 = m2m_rows_[p], sum_rows0 = m2m_sum_rows_[p];
+            int bkind = m2m_pref_[p], brows = bkind ? sum_rows0 : rows0;
             for (int kind : {0, 1, 2})
                 for (int rows : {1, 2, 4, 8, 16, 32, 64}) {
                     if (rows > nth_[p] && rows != 1) continue;
@@ -2437,14 +2454,15 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
                                                                     : m2m_sum_smem<float>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])) + 1024
                                              : static_cast<size_t>(8) * rows * nph_[p + 1] * 2 * csize;
                     if (need > static_cast<size_t>(dev_smem) || (!kind && rows > 16)) continue;
-                    m2m_rows_[p] = rows;
+                    (kind ? m2m_sum_rows_ : m2m_rows_)[p] = rows;
                     m2m_pref_[p] = kind;
                     const float t = timed([&] {
                         if (precision_ == kFp64) far_m2m<double, false>(f64_, p, s); else far_m2m<float, false>(f32_, p, s);
                     });
                     if (t < bt) { bt = t; brows = rows; bkind = kind; }
                 }
-            m2m_rows_[p] = brows;
+            m2m_rows_[p] = bkind ? rows0 : brows;
+            m2m_sum_rows_[p] = bkind ? brows : sum_rows0;
             m2m_pref_[p] = bkind;
             r.m2m_rows[p] = brows;
             if (n_l2l_pairs_[p]) {
@@ -2557,7 +2575,7 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
         if (m2m_pref_[p]) r.m2m_staged |= 1 << (m2m_pref_[p] == 2 ? 16 + p : p);
         if (l2l_pref_[p]) r.l2l_staged |= 1 << (l2l_pref_[p] == 3 ? 24 + p : l2l_pref_[p] == 2 ? 16 + p : p);
     }
-    for (int p = lmin_; p < lmax_; ++p) r.m2m_rows[p] = m2m_rows_[p];
+    for (int p = lmin_; p < lmax_; ++p) r.m2m_rows[p] = (m2m_pref_[p] ? m2m_sum_rows_ : m2m_rows_)[p];
     if (r.multi_rows_fast == 0 && m_m2m_rows_fast_ < 0) r.multi_rows_fast = -1;
     // restore the local patterns, drop captured graphs
     for (size_t i = 0; i < saved.size(); ++i)
