@@ -409,6 +409,10 @@ private:
     // xt_ -> yfar_, ynear_; krylov: a product of a solve (see run_near)
     void enqueue_core(cudaStream_t s, int prec, bool tr, bool krylov = false);
     void launch_core(cudaStream_t s, int prec, bool tr, bool krylov);
+    template <class R> bool m2m_windowed(const FarField<R>& F, int p) const;
+    template <class R> bool l2l_windowed(const FarField<R>& F, int p) const;
+    template <class R> bool multi_rows_fast() const;
+    template <class R> int multi_l2l_pairs() const;
     template <class R> void run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage);
     void run_far_multi(int nr, cudaStream_t s, int stage, int prec);
     void run_near_multi(int nr, cudaStream_t s);

@@ -35,6 +35,7 @@
 #include "kernels_near.cuh"
 #include "kernels_tables.cuh"
 #include "kernels_tc.cuh"
+#include "launch_rules.hpp"
 #include "zmath.cuh"
 
 namespace mlfma {
@@ -711,9 +712,9 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         F.l2t = upload(dn);
     }
     // Shared-memory limits.
-    size_t m2m_smem = 1, l2l_smem = 1;
+    size_t m2m_need = 1, l2l_smem = 1;
     for (int p = lmin_; p < lmax_; ++p) {
-        m2m_smem = std::max(m2m_smem, static_cast<size_t>(8) * m2m_rows(nth_[p], nph_[p]) * nph_[p + 1] * 2 * sizeof(C));
+        m2m_need = std::max(m2m_need, m2m_smem(m2m_rows(nth_[p], nph_[p]), nph_[p + 1], sizeof(C)));
         l2l_smem = std::max(l2l_smem, static_cast<size_t>(nth_[p]) * nph_[p + 1] * 2 * sizeof(C));
     }
     int dev_smem = 0;
@@ -721,7 +722,7 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
     const size_t s2m_smem = static_cast<size_t>(std::max(1, max_src_)) * sizeof(C);
     // k_l2t_half (complex-float far field) stages a leaf's local pattern twice
     const size_t l2t_smem = 2 * sizeof(C) * static_cast<size_t>(max_leaf_ndir_);
-    if (m2m_smem > static_cast<size_t>(dev_smem) || l2l_smem > static_cast<size_t>(dev_smem) ||
+    if (m2m_need > static_cast<size_t>(dev_smem) || l2l_smem > static_cast<size_t>(dev_smem) ||
         s2m_smem > static_cast<size_t>(dev_smem) ||
         (!std::is_same<R, double>::value && l2t_smem > static_cast<size_t>(dev_smem)))
         return "angular grid or leaf too large for the kernels' shared memory";
@@ -822,10 +823,9 @@ std::string DeviceOp::setup_far(const Plan& plan, FarField<R>& F, const double2*
         MLFMA_CK(dyn(reinterpret_cast<const void*>(k_l2l_m<R, 32, 2>)));
         for (int p = lmin_; p < lmax_; ++p) {
             const size_t m2m1 = static_cast<size_t>(nph_[p + 1]) * 32 * m2m_rpl<R>() * sizeof(C);
-            const size_t l2l1 = static_cast<size_t>(nth_[p]) * 2 * 1 * 64 * sizeof(C) +
-                                static_cast<size_t>(nth_[p + 1]) * dn_w_[p] * (sizeof(R) + 2 * sizeof(int));
+            const size_t l2l1 = l2l_m_smem(1, nth_[p], nth_[p + 1], dn_w_[p], sizeof(C));
             // (the static stencil staging takes at most 11 KB)
-            if (m2m1 + 11264 > static_cast<size_t>(dev_smem) || l2l1 + 1024 > static_cast<size_t>(dev_smem) ||
+            if (m2m1 + 11264 > static_cast<size_t>(dev_smem) || l2l1 + kSmemStatic > static_cast<size_t>(dev_smem) ||
                 nph_[p] > kM2MOut * kInterpWarps)
                 return "angular grid too large for the many-right-hand-side interpolation kernels";
         }
@@ -1231,9 +1231,9 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
 #undef MLFMA_M2M_SUM
         return;
     }
-    rows = m2m_rows_[p];
+    rows = m2m_fit_rows(m2m_rows_[p], nph_[p + 1], sizeof(C), dev_smem_);
     grid.y = (nth_[p] + rows - 1) / rows;
-    const size_t smem = static_cast<size_t>(8) * rows * nph_[p + 1] * 2 * sizeof(C);
+    const size_t smem = m2m_smem(rows, nph_[p + 1], sizeof(C));
     switch (up_w_[p]) {
         case 2: launch_k(pdl, k_m2m<R, 2, TR>, grid, 128, smem, s, F.lv_dev, T, rows); break;
         case 4: launch_k(pdl, k_m2m<R, 4, TR>, grid, 128, smem, s, F.lv_dev, T, rows); break;
@@ -1924,6 +1924,31 @@ void by_columns(int nr, F f) {
     else f(std::integral_constant<int, 4>());
 }
 
+// Transitions that the windowed kernels take (kernels_multi.cuh); the others run
+// k_m2m_m and k_l2l_m.
+template <class R>
+bool DeviceOp::m2m_windowed(const FarField<R>& F, int p) const {
+    return std::is_same<R, double>::value && F.trans[p].win_up && up_w_[p] == 6 &&
+           m2m_w_smem<R>(nph_[p + 1]) <= kWinSmem && precision_ == kFp64;
+}
+template <class R>
+bool DeviceOp::l2l_windowed(const FarField<R>& F, int p) const {
+    return F.trans[p].win_dn && l2l_w_smem<R>(nth_[p], nth_[p + 1], 1) <= kWinSmem &&
+           (std::is_same<R, float>::value || precision_ == kFp64);
+}
+// Grid order of k_m2m_m and column pairs of k_l2l_m: the tuner times them in the
+// operator's own precision, and a mixed operator's FP64 far field keeps its own.
+template <class R>
+bool DeviceOp::multi_rows_fast() const {
+    const bool own = std::is_same<R, double>::value == (precision_ == kFp64);
+    return own && m_m2m_rows_fast_ >= 0 ? m_m2m_rows_fast_ != 0 : m2m_rows_fast<R>();
+}
+template <class R>
+int DeviceOp::multi_l2l_pairs() const {
+    const bool own = std::is_same<R, double>::value == (precision_ == kFp64);
+    return own && m_l2l_pairs_ > 0 ? m_l2l_pairs_ : l2l_pairs<R>();
+}
+
 // stage: -1 all, 0 S2M, 1 M2M, 2 M2L, 3 L2L, 4 L2T.
 template <class R>
 void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage) {
@@ -1942,16 +1967,16 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
         for (int p = lmax_ - 1; p >= lmin_; --p) {
             if (npar_[p] == 0) continue;
             if constexpr (std::is_same<R, double>::value) {
-                const size_t wsm = sizeof(C) * nph_[p + 1] * kWinRows * 32;
-                if (F.trans[p].win_up && up_w_[p] == 6 && wsm <= kWinSmem && precision_ == kFp64) {
+                if (m2m_windowed(F, p)) {
                     const int ng = (nth_[p] + kWinRows - 1) / kWinRows;
-                    k_m2m_w<6><<<static_cast<unsigned>(npar_[p]) * ng * ((nr + 15) / 16), kInterpThreads, wsm, s>>>(
-                        F.lv_dev, F.trans[p], nr, ng);
+                    k_m2m_w<6><<<static_cast<unsigned>(npar_[p]) * ng * ((nr + 15) / 16), kInterpThreads,
+                                 m2m_w_smem<R>(nph_[p + 1]), s>>>(F.lv_dev, F.trans[p], nr, ng);
                     continue;
                 }
             }
             constexpr int rc = 16 * m2m_rpl<R>();
-            const int rows_fast = m_m2m_rows_fast_ < 0 ? (m2m_rows_fast<R>() ? 1 : 0) : m_m2m_rows_fast_;
+            // (tuned: of the operator's own precision; a grid's third extent is at most 65,535)
+            const int rows_fast = multi_rows_fast<R>() && npar_[p] <= 65535;
             const dim3 grid = rows_fast ? dim3(nth_[p], (nr + rc - 1) / rc, npar_[p])
                                         : dim3(npar_[p], nth_[p], (nr + rc - 1) / rc);
             const size_t smem = static_cast<size_t>(nph_[p + 1]) * 32 * m2m_rpl<R>() * sizeof(C);
@@ -1987,13 +2012,8 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
             if (!g) continue;
             // complex float: two right-hand sides a lane (each weight read serves
             // both) where the tile still leaves room for two blocks on an SM
-            auto wsm = [&](int rpl) {
-                return sizeof(C) * nth_[p] * 2 * kWinCols * 32 * rpl +
-                       static_cast<size_t>((nth_[p + 1] + kWinCols - 1) / kWinCols) * kWinTapsTh *
-                           (kWinCols * sizeof(R) + sizeof(int2));
-            };
-            if (F.trans[p].win_dn && wsm(1) <= kWinSmem &&
-                (std::is_same<R, float>::value || precision_ == kFp64)) {
+            auto wsm = [&](int rpl) { return l2l_w_smem<R>(nth_[p], nth_[p + 1], rpl); };
+            if (l2l_windowed(F, p)) {
                 const int ng = (nph_[p + 1] / 2 + kWinCols - 1) / kWinCols;
                 if constexpr (std::is_same<R, float>::value)
                     if (nr > 16 && wsm(2) <= kWinSmem) {
@@ -2005,10 +2025,9 @@ void DeviceOp::run_far_multi_t(FarField<R>& F, int nr, cudaStream_t s, int stage
                                                                                          l2l_pairs_[p], nr);
                 continue;
             }
-            const int pairs = m_l2l_pairs_ > 0 ? m_l2l_pairs_ : l2l_pairs<R>();
+            const int pairs = l2l_m_fit_pairs(multi_l2l_pairs<R>(), nth_[p], nth_[p + 1], dn_w_[p], sizeof(C), dev_smem_);
             const dim3 grid(g, (nph_[p + 1] / 2 + pairs - 1) / pairs, (nr + kRc - 1) / kRc);
-            const size_t smem = static_cast<size_t>(nth_[p]) * 2 * pairs * 64 * sizeof(C) +
-                                static_cast<size_t>(nth_[p + 1]) * dn_w_[p] * (sizeof(R) + 2 * sizeof(int));
+            const size_t smem = l2l_m_smem(pairs, nth_[p], nth_[p + 1], dn_w_[p], sizeof(C));
             const DevTransT<R>& T = F.trans[p];
 #define MLFMA_L2L_M(WW)                                                                                    \
     (pairs == 1 ? k_l2l_m<R, WW, 1><<<grid, kInterpThreads, smem, s>>>(F.lv_dev, T, l2l_pairs_[p], nr)     \
@@ -2430,10 +2449,12 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
     if (nr == 1) {
         auto product = [&] { enqueue_core(s, precision_, false); };
         r.before_ms = timed(product);
-        // M2L: directions per block
+        // M2L: directions per block, where a level reads it (families do not)
         float best = 1e30f;
         int best_chunk = m2l_chunk_;
-        for (int chunk : {32, 64, 96, 128}) {  // k_m2l runs 128 threads: one direction each
+        bool reads_chunk = !m2l_staged_;
+        for (int l = lmin_; l <= lmax_; ++l) reads_chunk = reads_chunk || (m2l_count_[l] && !m2l_fam_count_[l]);
+        if (reads_chunk) for (int chunk : {32, 64, 96, 128}) {  // k_m2l runs 128 threads: one direction each
             build_m2l_items(chunk);
             const float t = timed([&] { run_far(xt_, s, 2, precision_, false); });
             if (t < best) { best = t; best_chunk = chunk; }
@@ -2452,7 +2473,7 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
                     if (rows > nth_[p] && rows != 1) continue;
                     const size_t need = kind ? (precision_ == kFp64 ? m2m_sum_smem<double>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])
                                                                     : m2m_sum_smem<float>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])) + 1024
-                                             : static_cast<size_t>(8) * rows * nph_[p + 1] * 2 * csize;
+                                             : m2m_smem(rows, nph_[p + 1], csize);
                     if (need > static_cast<size_t>(dev_smem) || (!kind && rows > 16)) continue;
                     (kind ? m2m_sum_rows_ : m2m_rows_)[p] = rows;
                     m2m_pref_[p] = kind;
@@ -2532,27 +2553,36 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
     } else {
         auto product = [&] { enqueue_multi(nr, s, precision_); };
         r.before_ms = timed(product);
-        float bt = 1e30f;
-        int border = m_m2m_rows_fast_;
-        for (int o : {0, 1}) {
-            m_m2m_rows_fast_ = o;
-            const float t = timed([&] { run_far_multi(nr, s, 1, precision_); });
-            if (t < bt) { bt = t; border = o; }
+        // each choice is timed only where a transition of the timed path reads it
+        // (the windowed and the tensor-core kernels do not); else it stays
+        bool reads_order = false, reads_pairs = false, two_fit = false;
+        for (int p = lmin_; p < lmax_; ++p) {
+            const bool f64 = precision_ == kFp64;
+            const bool up = f64 ? m2m_windowed(f64_, p) : m2m_windowed(f32_, p) || (tc_mode_ & 2);
+            const bool dn = f64 ? l2l_windowed(f64_, p) : l2l_windowed(f32_, p) || (tc_mode_ & 8);
+            reads_order = reads_order || (npar_[p] && !up);
+            if (!n_l2l_pairs_[p] || dn) continue;
+            reads_pairs = true;
+            two_fit = two_fit || l2l_m_fit_pairs(2, nth_[p], nth_[p + 1], dn_w_[p], csize, dev_smem_) == 2;
         }
+        float bt = 1e30f;
+        int border = precision_ == kFp64 ? multi_rows_fast<double>() : multi_rows_fast<float>();
+        if (reads_order)
+            for (int o : {0, 1}) {
+                m_m2m_rows_fast_ = o;
+                const float t = timed([&] { run_far_multi(nr, s, 1, precision_); });
+                if (t < bt) { bt = t; border = o; }
+            }
         m_m2m_rows_fast_ = border;
         bt = 1e30f;
-        int bpairs = m_l2l_pairs_;
-        for (int q : {1, 2}) {
-            bool fits = true;
-            for (int p = lmin_; p < lmax_; ++p)
-                if (static_cast<size_t>(nth_[p]) * 2 * q * 64 * csize + static_cast<size_t>(nth_[p + 1]) * dn_w_[p] * 16 + 1024 >
-                    static_cast<size_t>(dev_smem))
-                    fits = false;
-            if (!fits) continue;
-            m_l2l_pairs_ = q;
-            const float t = timed([&] { run_far_multi(nr, s, 3, precision_); });
-            if (t < bt) { bt = t; bpairs = q; }
-        }
+        int bpairs = precision_ == kFp64 ? multi_l2l_pairs<double>() : multi_l2l_pairs<float>();
+        if (reads_pairs)
+            for (int q : {1, 2}) {
+                if (q == 2 && !two_fit) continue;
+                m_l2l_pairs_ = q;
+                const float t = timed([&] { run_far_multi(nr, s, 3, precision_); });
+                if (t < bt) { bt = t; bpairs = q; }
+            }
         m_l2l_pairs_ = bpairs;
         r.multi_rows_fast = border;
         r.multi_l2l_pairs = bpairs;

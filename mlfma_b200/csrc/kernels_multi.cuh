@@ -500,6 +500,17 @@ k_l2l_m(const DevLevelT<R>* __restrict__ lvs, DevTransT<R> T, const int2* __rest
 // kernels.  Measured (M2M, L2L): r = 2 sphere x 64, FP64, 605 and 1,250 us before,
 // 448 and 915 now; 12,347 dipoles x 17, complex float, L2L 245 -> 149 us.
 
+// Shared memory of the two tiles.
+template <class R>
+size_t m2m_w_smem(int child_nph) {
+    return sizeof(typename Cx<R>::T) * child_nph * kWinRows * 32;
+}
+template <class R>
+size_t l2l_w_smem(int parent_nth, int child_nth, int rpl) {
+    return sizeof(typename Cx<R>::T) * parent_nth * 2 * kWinCols * 32 * rpl +
+           static_cast<size_t>((child_nth + kWinCols - 1) / kWinCols) * kWinTapsTh * (kWinCols * sizeof(R) + sizeof(int2));
+}
+
 // Parent outgoing patterns, complex double (complex float, whose sums keep the
 // folded weights' rounding, was slower this way: 161 -> 244 us).  Children
 // shifted and summed at every tap of the union first, then one theta pass with

@@ -1,0 +1,47 @@
+// CPU check of the launch rules (launch_rules.hpp): over grids of every size that
+// setup accepts and both element sizes, the chosen tile fits the block's shared
+// memory wherever the smallest one does, is never larger than asked for, and is
+// not given up while it fits.  Run by tests/test_launch_rules.py.
+#include "launch_rules.hpp"
+
+#include <cstdio>
+using namespace mlfma;
+
+static int bad = 0;
+#define CHECK(c)                                                            \
+    do {                                                                    \
+        if (!(c) && bad++ < 20) std::printf("line %d: %s\n", __LINE__, #c); \
+    } while (0)
+
+int main() {
+    const size_t limit = 232448;  // opt-in shared memory of a block
+    for (size_t elem : {8u, 16u})
+        for (int nth = 4; nth <= 160; ++nth) {
+            const int nph = 2 * nth;
+            // child by child: rows as tuned with either element size
+            for (int rows : {1, 2, 3, 4, 8, 16}) {
+                const int got = m2m_fit_rows(rows, nph, elem, limit);
+                CHECK(got >= 1 && got <= rows);
+                CHECK(m2m_smem(got, nph, elem) <= limit || got == 1);
+                if (m2m_smem(rows, nph, elem) <= limit) CHECK(got == rows);
+            }
+            for (int w : {8, 12, 16, 24, 32})
+                for (int cth = 4; cth <= nth; ++cth) {
+                    if (l2l_m_smem(1, nth, cth, w, elem) + kSmemStatic > limit) continue;  // refused at setup
+                    for (int pairs : {1, 2}) {
+                        const int got = l2l_m_fit_pairs(pairs, nth, cth, w, elem, limit);
+                        CHECK(got >= 1 && got <= pairs);
+                        CHECK(l2l_m_smem(got, nth, cth, w, elem) + kSmemStatic <= limit);
+                        if (l2l_m_smem(pairs, nth, cth, w, elem) + kSmemStatic <= limit) CHECK(got == pairs);
+                    }
+                }
+        }
+    // the grids of a root of 16 wavelengths, tuned in complex float: two pairs of
+    // 58 rows and 16 rows of 68 columns fit 8-byte elements and not 16-byte ones
+    CHECK(l2l_m_fit_pairs(2, 58, 34, 12, 8, limit) == 2);
+    CHECK(l2l_m_fit_pairs(2, 58, 34, 12, 16, limit) == 1);
+    CHECK(m2m_fit_rows(16, 68, 8, limit) == 16);
+    CHECK(m2m_fit_rows(16, 68, 16, limit) == 8);
+    std::printf(bad ? "%d FAILED\n" : "ALL OK\n", bad);
+    return bad != 0;
+}
