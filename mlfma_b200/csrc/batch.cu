@@ -55,6 +55,7 @@ namespace {
 // Records every operator's product, reading d_x and writing d_y (packed), as
 // parallel branches forked from and joined back into b->stream.
 int capture(mlfma_batch_s* b) {
+    cudaGetLastError();  // an earlier call's error is not this capture's
     B_CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaEventRecord(b->fork, b->stream);
     for (size_t i = 0; i < b->ops.size(); ++i) {
@@ -74,7 +75,9 @@ int capture(mlfma_batch_s* b) {
                                                            " failed: " + cudaGetErrorString(le));
         }
     }
+    const std::string refused = mlfma::DeviceOp::launch_status();  // (a refused launch is missing from the graph)
     B_CK(cudaStreamEndCapture(b->stream, &b->graph));
+    if (!refused.empty()) return mlfma_internal_fail(MLFMA_ERR_CUDA, refused);
     B_CK(cudaGraphInstantiate(&b->exec, b->graph, cudaGraphInstantiateFlagUseNodePriority));
     return MLFMA_OK;
 }

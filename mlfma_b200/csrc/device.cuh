@@ -293,10 +293,15 @@ public:
     // results since then are not valid); read after the stream is synchronised.
     std::string device_error() const;
 
-    // Operator on tree-ordered device vectors (used by the solver).
-    void apply_tree(const double2* xt, double2* yt, cudaStream_t s, int prec = -1, bool adj = false);
+    // Non-empty when a kernel launch of this thread was refused since the last
+    // call (the launches themselves return nothing).
+    static std::string launch_status();
+
+    // Operator on tree-ordered device vectors (used by the solver); a message
+    // when a launch was refused.
+    std::string apply_tree(const double2* xt, double2* yt, cudaStream_t s, int prec = -1, bool adj = false);
     // Same, never capturing a graph (launches the captured one if it exists).
-    void apply_tree_direct(const double2* xt, double2* yt, cudaStream_t s, int prec = -1, bool adj = false);
+    std::string apply_tree_direct(const double2* xt, double2* yt, cudaStream_t s, int prec = -1, bool adj = false);
     // The product of what is already in the operator's input buffer (xt_buffer(),
     // tree order; for the adjoint it holds conj(x)) into yt, with plain
     // launches (for capture into a solver's step graph).
@@ -318,7 +323,7 @@ public:
     std::string matvec_multi_device(const double2* x, double2* y, int nr, bool accumulate, cudaStream_t stream,
                                     int prec = -1);
     // Tree order, right-hand side innermost ([n][nr]), for the solver.
-    void apply_tree_multi(const double2* xt, double2* yt, int nr, cudaStream_t s, int prec = -1);
+    std::string apply_tree_multi(const double2* xt, double2* yt, int nr, cudaStream_t s, int prec = -1);
     int max_rhs() const { return max_rhs_; }
 
     // One product on caller-order device vectors, recorded on stream s with

@@ -487,8 +487,12 @@ std::string Gmres::step_graph(DeviceOp& op, int prec) {
                                                                                           pass, swnorm_);
         k_step_update<<<nblk(n, kUpdThreads), kUpdThreads, 0, s>>>(st, Q_, n, tco_, w_, npart2_, hcols_, ldh, pass);
     }
+    const std::string refused = DeviceOp::launch_status();  // (a refused launch is missing from the graph)
     const cudaError_t ce = cudaStreamEndCapture(s, &sg_);
-    if (ce != cudaSuccess) return std::string("step capture: ") + cudaGetErrorString(ce);
+    if (ce != cudaSuccess || !refused.empty()) {
+        cudaGetLastError();
+        return "step capture: " + (refused.empty() ? std::string(cudaGetErrorString(ce)) : refused);
+    }
     GM_CK(cudaGraphInstantiate(&sgx_, sg_, cudaGraphInstantiateFlagUseNodePriority));
     sg_op_ = &op;
     sg_prec_ = prec;
@@ -539,8 +543,8 @@ void Gmres::release_outer() {
     on_ = ocap_ = 0;
 }
 
-void Gmres::apply(DeviceOp& op, const double2* x, double2* y, cudaStream_t s, int prec) {
-    if (external_) op.apply_tree_direct(x, y, s, prec, adj_); else op.apply_tree(x, y, s, prec, adj_);
+std::string Gmres::apply(DeviceOp& op, const double2* x, double2* y, cudaStream_t s, int prec) {
+    return external_ ? op.apply_tree_direct(x, y, s, prec, adj_) : op.apply_tree(x, y, s, prec, adj_);
 }
 
 // ------------------------------------------------------------ fixed workspace
@@ -688,10 +692,11 @@ std::string Gmres::cycles(DeviceOp& op, int prec, const SolveOpts& o, double bno
         } else {
             if (pc_) {  // x_ holds u with x = M^{-1} u
                 op.bj_apply(x_, tq_, s);
-                apply(op, tq_, w_, s, prec);
+                err = apply(op, tq_, w_, s, prec);
             } else {
-                apply(op, x_, w_, s, prec);
+                err = apply(op, x_, w_, s, prec);
             }
+            if (!err.empty()) return err;
             k_sub<<<nblk(n, 256), 256, 0, s>>>(b_, w_, r_, n);
             err = norm(r_, s, &beta);
             if (!err.empty()) return err;
@@ -781,10 +786,11 @@ std::string Gmres::cycles(DeviceOp& op, int prec, const SolveOpts& o, double bno
                 double2* qk = Q_ + static_cast<long long>(k) * n;
                 if (pc_) {  // w = A M^{-1} q_k
                     op.bj_apply(qk, tq_, s);
-                    apply(op, tq_, w_, s, prec);
+                    err = apply(op, tq_, w_, s, prec);
                 } else {
-                    apply(op, qk, w_, s, prec);  // w = A q_k
+                    err = apply(op, qk, w_, s, prec);  // w = A q_k
                 }
+                if (!err.empty()) return err;
                 err = cgs_pass(k + 1, s, false);
                 if (!err.empty()) return err;
                 err = cgs_pass(k + 1, s, true);
@@ -838,6 +844,7 @@ std::string Gmres::cycles(DeviceOp& op, int prec, const SolveOpts& o, double bno
 std::string Gmres::solve(DeviceOp& op, const double2* d_b_user, double2* d_x_user, const SolveOpts& o,
                          SolveResult* res) {
     if (o.adjoint && op.ref_compat()) return "arg:the adjoint needs ref_compat = 0";
+    cudaGetLastError();  // an earlier call's error is not this solve's
     adj_ = o.adjoint != 0;
     pc_ = o.precond != 0;
     if (o.inner) {
@@ -883,7 +890,8 @@ std::string Gmres::solve(DeviceOp& op, const double2* d_b_user, double2* d_x_use
                  &converged);
     if (!err.empty()) return err;
     // True residual.
-    apply(op, x_, w_, s);
+    err = apply(op, x_, w_, s);
+    if (!err.empty()) return err;
     k_sub<<<nblk(n, 256), 256, 0, s>>>(b_, w_, r_, n);
     double rn;
     err = norm(r_, s, &rn);
@@ -944,7 +952,8 @@ std::string Gmres::solve_refined(DeviceOp& op, const double2* d_b_user, double2*
         res->iterations += it;
         // x += d ; r = b - A64 x  (FP64)
         k_axpy1<<<nblk(n, 256), 256, 0, s>>>(x_, xo_, n);
-        apply(op, xo_, w_, s, kFp64);
+        err = apply(op, xo_, w_, s, kFp64);
+        if (!err.empty()) return err;
         k_sub<<<nblk(n, 256), 256, 0, s>>>(bo_, w_, b_, n);
         ++res->refinements;
         err = norm(b_, s, &rn);
@@ -1045,7 +1054,8 @@ std::string Gmres::solve_flexible(DeviceOp& op, const double2* d_b_user, double2
             res->iterations += it;
             GM_CK(cudaMemcpyAsync(zk, x_, sizeof(double2) * n, cudaMemcpyDeviceToDevice, s));
             // w = A z_k in FP64, orthogonalised against v_0..v_k
-            apply(op, zk, wo_, s, kFp64);
+            err = apply(op, zk, wo_, s, kFp64);
+            if (!err.empty()) return err;
             ++res->refinements;
             cgs2(k + 1);
             k_norm2<<<nch, kDotThreads, 0, s>>>(wo_, n, npartial_);
@@ -1098,7 +1108,8 @@ std::string Gmres::solve_flexible(DeviceOp& op, const double2* d_b_user, double2
         GM_CK(cudaMemcpyAsync(to_, yd.data(), sizeof(double2) * k, cudaMemcpyHostToDevice, s));
         k_sub_qh<<<nblk(n, 256), 256, 0, s>>>(Z_, n, k, to_, xf_, n);
         // true FP64 residual
-        apply(op, xf_, wo_, s, kFp64);
+        err = apply(op, xf_, wo_, s, kFp64);
+        if (!err.empty()) return err;
         k_sub<<<nblk(n, 256), 256, 0, s>>>(bf_, wo_, r_, n);
         err = norm(r_, s, &beta);
         if (!err.empty()) return err;

@@ -53,7 +53,7 @@ public:
     std::string use_static_workspace(int n, int ncols, int extra = 0);
 
 private:
-    void apply(DeviceOp& op, const double2* x, double2* y, cudaStream_t s, int prec = -1);
+    std::string apply(DeviceOp& op, const double2* x, double2* y, cudaStream_t s, int prec = -1);
     // Restarted GMRES on A(prec) x_ = b_ from x_ = 0 until the estimated
     // residual norm is at most tol_abs or max_iter iterations have run.
     std::string cycles(DeviceOp& op, int prec, const SolveOpts& o, double bnorm, double tol_abs, int max_iter,

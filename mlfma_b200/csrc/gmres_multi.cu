@@ -247,7 +247,8 @@ std::string GmresMulti::cycles(DeviceOp& op, int prec, int restart, int max_iter
             GMM_CK(cudaMemcpyAsync(r_, b_, sizeof(double2) * ld, cudaMemcpyDeviceToDevice, s));
             beta = bnorm;
         } else {
-            op.apply_tree_multi(x_, w_, nr, s, prec);
+            err = op.apply_tree_multi(x_, w_, nr, s, prec);
+            if (!err.empty()) return err;
             k_msub<<<nblk(ld, 256), 256, 0, s>>>(b_, w_, r_, ld);
             err = norms(r_, s, beta);
             if (!err.empty()) return err;
@@ -276,7 +277,8 @@ std::string GmresMulti::cycles(DeviceOp& op, int prec, int restart, int max_iter
         int k = 0;
         for (; k < m && total < max_iter && nact > 0; ++k) {
             double2* qk = Q_ + static_cast<long long>(k) * ld;
-            op.apply_tree_multi(qk, w_, nr, s, prec);
+            err = op.apply_tree_multi(qk, w_, nr, s, prec);
+            if (!err.empty()) return err;
             cgs_pass(k + 1, s, false);
             cgs_pass(k + 1, s, true);
             k_mnorm2<<<nchunks_, kThreads, 0, s>>>(w_, n, nr, npartial_);
@@ -358,6 +360,7 @@ std::string GmresMulti::solve(DeviceOp& op, int nr, const double2* d_b_user, dou
     if (nr < 1 || nr > op.max_rhs()) return "arg:nrhs must be between 1 and the operator's max_rhs";
     const int m = o.restart > 0 ? o.restart : o.max_iter;
     if (m < 1 || o.max_iter < 1) return "arg:max_iter and restart must be positive";
+    cudaGetLastError();  // an earlier call's error is not this solve's
     if (o.flexible) return solve_flexible(op, nr, d_b_user, d_x_user, o, res);
     std::string err = ensure(n, nr, m + 1);
     if (!err.empty()) return err;
@@ -383,7 +386,8 @@ std::string GmresMulti::solve(DeviceOp& op, int nr, const double2* d_b_user, dou
         err = cycles(op, -1, o.restart, o.max_iter, bnorm, tol_abs, done, iters, est);
         if (!err.empty()) return err;
         GMM_CK(cudaMemcpyAsync(xo_, x_, sizeof(double2) * ld, cudaMemcpyDeviceToDevice, s));
-        op.apply_tree_multi(xo_, w_, nr, s, -1);
+        err = op.apply_tree_multi(xo_, w_, nr, s, -1);
+        if (!err.empty()) return err;
         k_msub<<<nblk(ld, 256), 256, 0, s>>>(bo_, w_, r_, ld);
         err = norms(r_, s, rn);
         if (!err.empty()) return err;
@@ -412,7 +416,8 @@ std::string GmresMulti::solve(DeviceOp& op, int nr, const double2* d_b_user, dou
             bool progress = false;
             for (int r = 0; r < nr; ++r) { iters[r] += it[r]; progress = progress || it[r] > 0; }
             k_maxpy<<<nblk(ld, 256), 256, 0, s>>>(x_, xo_, ld);  // frozen columns have x_ = 0
-            op.apply_tree_multi(xo_, w_, nr, s, kFp64);
+            err = op.apply_tree_multi(xo_, w_, nr, s, kFp64);
+            if (!err.empty()) return err;
             k_msub<<<nblk(ld, 256), 256, 0, s>>>(bo_, w_, b_, ld);
             err = norms(b_, s, rn);
             if (!err.empty()) return err;
@@ -526,7 +531,8 @@ std::string GmresMulti::solve_flexible(DeviceOp& op, int nr, const double2* d_b_
             if (!err.empty()) return err;
             GMM_CK(cudaMemcpyAsync(zk, x_, sizeof(double2) * ld, cudaMemcpyDeviceToDevice, s));
             // w = A z_k in FP64, orthogonalised against v_0..v_k of its column
-            op.apply_tree_multi(zk, w_, nr, s, kFp64);
+            err = op.apply_tree_multi(zk, w_, nr, s, kFp64);
+            if (!err.empty()) return err;
             cgs_pass_q(V_, w_, k + 1, s, h_, false);
             cgs_pass_q(V_, w_, k + 1, s, h_, true);
             k_mnorm2<<<nchunks_, kThreads, 0, s>>>(w_, n, nr, npartial_);
@@ -591,7 +597,8 @@ std::string GmresMulti::solve_flexible(DeviceOp& op, int nr, const double2* d_b_
             k_msub_qh<<<nblk(ld, 256), 256, 0, s>>>(Z_, ld, kmax, y_, xo_, ld, nr);
         }
         // true FP64 residual
-        op.apply_tree_multi(xo_, w_, nr, s, kFp64);
+        err = op.apply_tree_multi(xo_, w_, nr, s, kFp64);
+        if (!err.empty()) return err;
         k_msub<<<nblk(ld, 256), 256, 0, s>>>(bo_, w_, r_, ld);
         err = norms(r_, s, beta);
         if (!err.empty()) return err;

@@ -1503,11 +1503,21 @@ void DeviceOp::enqueue_core(cudaStream_t s, int prec, bool tr, bool krylov) {
 std::string DeviceOp::ensure_graph(int prec, bool tr, bool krylov) {
     const int t = tr ? 1 : 0, k = krylov && precision_ != kFp64 ? 1 : 0;
     if (graph_exec_[prec][t][k] || !use_graph_) return {};
+    cudaGraph_t& g = graph_[prec][t][k];
+    cudaGetLastError();  // an earlier caller's error is not this capture's
     MLFMA_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     enqueue_core(stream_, prec, tr, krylov);
-    MLFMA_CK(cudaStreamEndCapture(stream_, &graph_[prec][t][k]));
-    MLFMA_CK(cudaGraphInstantiate(&graph_exec_[prec][t][k], graph_[prec][t][k], cudaGraphInstantiateFlagUseNodePriority));
-    return {};
+    // a launch that was refused is missing from the graph: it is not kept
+    const std::string refused = launch_status();
+    cudaError_t e = cudaStreamEndCapture(stream_, &g);
+    if (e == cudaSuccess && refused.empty())
+        e = cudaGraphInstantiate(&graph_exec_[prec][t][k], g, cudaGraphInstantiateFlagUseNodePriority);
+    if (e == cudaSuccess && refused.empty()) return {};
+    cudaGetLastError();
+    if (g) cudaGraphDestroy(g);
+    g = nullptr;
+    graph_exec_[prec][t][k] = nullptr;
+    return refused.empty() ? std::string("capture of a product: ") + cudaGetErrorString(e) : refused;
 }
 
 void DeviceOp::launch_core(cudaStream_t s, int prec, bool tr, bool krylov) {
@@ -1532,15 +1542,17 @@ std::string DeviceOp::set_loads(const double2* z_user) {
     return {};
 }
 
+// Non-empty when a launch since the last call was refused: its output is missing.
+std::string DeviceOp::launch_status() {
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? std::string() : std::string("a kernel launch was refused: ") + cudaGetErrorString(e);
+}
+
 // Tree-ordered y = A x (adj: y = A^H x = conj(A^T conj(x))), loads included.
-void DeviceOp::apply_tree(const double2* xt, double2* yt, cudaStream_t s, int prec, bool adj) {
+std::string DeviceOp::apply_tree(const double2* xt, double2* yt, cudaStream_t s, int prec, bool adj) {
     if (prec < 0) prec = precision_;
     if (!ensure_graph(prec, adj, true).empty()) use_graph_ = false;
-    if (adj) k_conj_copy<<<blocks_for(n_, 256), 256, 0, s>>>(xt, xt_, n_);
-    else if (xt != xt_) cudaMemcpyAsync(xt_, xt, sizeof(double2) * n_, cudaMemcpyDeviceToDevice, s);
-    launch_core(s, prec, adj, true);
-    k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, nullptr, yt, n_, ck_, 0, xt_,
-                                                 has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
+    return apply_tree_direct(xt, yt, s, prec, adj);
 }
 
 void DeviceOp::enqueue_apply_from_input(double2* yt, cudaStream_t s, int prec, bool adj) {
@@ -1550,13 +1562,14 @@ void DeviceOp::enqueue_apply_from_input(double2* yt, cudaStream_t s, int prec, b
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
 }
 
-void DeviceOp::apply_tree_direct(const double2* xt, double2* yt, cudaStream_t s, int prec, bool adj) {
+std::string DeviceOp::apply_tree_direct(const double2* xt, double2* yt, cudaStream_t s, int prec, bool adj) {
     if (prec < 0) prec = precision_;
     if (adj) k_conj_copy<<<blocks_for(n_, 256), 256, 0, s>>>(xt, xt_, n_);
     else if (xt != xt_) cudaMemcpyAsync(xt_, xt, sizeof(double2) * n_, cudaMemcpyDeviceToDevice, s);
     launch_core(s, prec, adj, true);
     k_finish<<<blocks_for(n_, 256), 256, 0, s>>>(yfar_, ynear_, nullptr, yt, n_, ck_, 0, xt_,
                                                  has_loads_ ? loads_ : nullptr, adj ? 1 : 0);
+    return launch_status();
 }
 
 std::string DeviceOp::matvec_device(const double2* x, double2* y, bool accumulate, cudaStream_t stream, int prec,
@@ -2091,13 +2104,14 @@ std::string DeviceOp::matvec_multi_device(const double2* x, double2* y, int nr, 
     return {};
 }
 
-void DeviceOp::apply_tree_multi(const double2* xt, double2* yt, int nr, cudaStream_t s, int prec) {
+std::string DeviceOp::apply_tree_multi(const double2* xt, double2* yt, int nr, cudaStream_t s, int prec) {
     if (prec < 0) prec = precision_;
     const long long tot = static_cast<long long>(n_) * nr;
     if (xt != xtm_) cudaMemcpyAsync(xtm_, xt, sizeof(double2) * tot, cudaMemcpyDeviceToDevice, s);
     enqueue_multi(nr, s, prec);
     k_finish_m<<<blocks_for(tot, 256), 256, 0, s>>>(yfarm_, ynearm_, nullptr, yt, n_, nr, ck_, 0, xtm_,
                                                      has_loads_ ? loads_ : nullptr);
+    return launch_status();
 }
 
 std::string DeviceOp::time_stages_multi(int nr, StageTimes* out) {
