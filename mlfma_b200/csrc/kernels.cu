@@ -1214,13 +1214,14 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
     using C = typename Cx<R>::T;
     if (npar_[p] == 0) return;
     const DevTransT<R>& T = F.trans[p];
-    int rows = m2m_sum_rows_[p];
-    dim3 grid(npar_[p], (nth_[p] + rows - 1) / rows);
-    const size_t ssum = m2m_sum_smem<R>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p]);
-    if (!TR && m2m_pref_[p] && ssum + 1024 <= static_cast<size_t>(dev_smem_)) {
+    const int sum_rows =
+        m2m_sum_fit_rows(m2m_sum_rows_[p], nth_[p + 1], nph_[p], nph_[p + 1], up_w_[p], sizeof(C), dev_smem_);
+    if (!TR && m2m_pref_[p] && sum_rows) {
         const bool cs = m2m_pref_[p] == 2;
+        const dim3 grid(npar_[p], (nth_[p] + sum_rows - 1) / sum_rows);
+        const size_t smem = m2m_sum_smem(sum_rows, nth_[p + 1], nph_[p], nph_[p + 1], up_w_[p], sizeof(C));
 #define MLFMA_M2M_SUM(WW) \
-    launch_k(pdl, cs ? k_m2m_sum<R, WW, true> : k_m2m_sum<R, WW, false>, grid, 256, ssum, s, T, rows)
+    launch_k(pdl, cs ? k_m2m_sum<R, WW, true> : k_m2m_sum<R, WW, false>, grid, 256, smem, s, T, sum_rows)
         switch (up_w_[p]) {
             case 2: MLFMA_M2M_SUM(2); break;
             case 4: MLFMA_M2M_SUM(4); break;
@@ -1231,8 +1232,8 @@ void DeviceOp::far_m2m(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
 #undef MLFMA_M2M_SUM
         return;
     }
-    rows = m2m_fit_rows(m2m_rows_[p], nph_[p + 1], sizeof(C), dev_smem_);
-    grid.y = (nth_[p] + rows - 1) / rows;
+    const int rows = m2m_fit_rows(m2m_rows_[p], nph_[p + 1], sizeof(C), dev_smem_);
+    const dim3 grid(npar_[p], (nth_[p] + rows - 1) / rows);
     const size_t smem = m2m_smem(rows, nph_[p + 1], sizeof(C));
     switch (up_w_[p]) {
         case 2: launch_k(pdl, k_m2m<R, 2, TR>, grid, 128, smem, s, F.lv_dev, T, rows); break;
@@ -1318,7 +1319,10 @@ void DeviceOp::far_l2l(FarField<R>& F, int p, cudaStream_t s, bool pdl) {
 #undef MLFMA_L2L_PIPE
         return;
     }
-    if (l2l_pref_[p] && l2l_pref_[p] != 3 && sst + 1024 <= static_cast<size_t>(dev_smem_)) {
+    // Where the tile does not fit, k_l2l is no slower: parents of 47 x 94 directions in
+    // FP64 115 us (staged without its stencils, which fits, 105; with an older staged
+    // kernel 124), 67 x 134 in complex float 114 us (158; 156).
+    if (l2l_pref_[p] && l2l_pref_[p] != 3 && sst + kSmemStatic <= static_cast<size_t>(dev_smem_)) {
         const bool cs = l2l_pref_[p] == 2;
 #define MLFMA_L2L_ST(WW)                                                                             \
     launch_k(pdl, cs ? k_l2l_st<R, WW, TR, true> : k_l2l_st<R, WW, TR, false>, g, 256, sst, s, T)
@@ -2485,10 +2489,9 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
             for (int kind : {0, 1, 2})
                 for (int rows : {1, 2, 4, 8, 16, 32, 64}) {
                     if (rows > nth_[p] && rows != 1) continue;
-                    const size_t need = kind ? (precision_ == kFp64 ? m2m_sum_smem<double>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])
-                                                                    : m2m_sum_smem<float>(nth_[p + 1], nph_[p], nph_[p + 1], rows, up_w_[p])) + 1024
-                                             : m2m_smem(rows, nph_[p + 1], csize);
-                    if (need > static_cast<size_t>(dev_smem) || (!kind && rows > 16)) continue;
+                    if (kind ? m2m_sum_fit_rows(rows, nth_[p + 1], nph_[p], nph_[p + 1], up_w_[p], csize, dev_smem) != rows
+                             : rows > 16 || m2m_smem(rows, nph_[p + 1], csize) > static_cast<size_t>(dev_smem))
+                        continue;
                     (kind ? m2m_sum_rows_ : m2m_rows_)[p] = rows;
                     m2m_pref_[p] = kind;
                     const float t = timed([&] {

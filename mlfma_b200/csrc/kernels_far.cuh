@@ -871,14 +871,6 @@ k_m2m_sum(DevTransT<R> T, int rows) {
     }
 }
 
-// Shared memory of k_m2m_sum for a tile of `rows` parent rows (bound: every
-// child row in the band).
-template <class R>
-size_t m2m_sum_smem(int child_nth, int parent_nph, int child_nph, int rows, int w) {
-    return static_cast<size_t>(child_nth + rows) * child_nph * 2 * sizeof(typename Cx<R>::T) +
-           static_cast<size_t>(rows + parent_nph) * w * (sizeof(R) + sizeof(int));
-}
-
 // L2L (and, POST, the transposed M2M) with the parent's local pattern, shifted
 // to the child's octant, staged in shared memory once per block: the same
 // arithmetic in the same order as k_l2l, every phi tap then reading shared

@@ -25,6 +25,19 @@ inline int m2m_fit_rows(int rows, int child_nph, size_t elem, size_t limit) {
     return rows;
 }
 
+// Aggregation with the children summed first (k_m2m_sum): the band of child rows
+// (bound: all of them), the theta pass's rows, and the stencils (w taps a row).
+inline size_t m2m_sum_smem(int rows, int child_nth, int parent_nph, int child_nph, int w, size_t elem) {
+    return static_cast<size_t>(child_nth + rows) * child_nph * 2 * elem +
+           static_cast<size_t>(rows + parent_nph) * w * (elem / 2 + sizeof(int));
+}
+// Parent rows per block: `rows`, halved until the tile fits; 0 where not even one
+// row does (k_m2m).
+inline int m2m_sum_fit_rows(int rows, int child_nth, int parent_nph, int child_nph, int w, size_t elem, size_t limit) {
+    while (rows >= 1 && m2m_sum_smem(rows, child_nth, parent_nph, child_nph, w, elem) + kSmemStatic > limit) rows /= 2;
+    return rows;
+}
+
 // Many-rhs anterpolation (k_l2l_m): `pairs` column pairs and the theta stencils.
 inline size_t l2l_m_smem(int pairs, int parent_nth, int child_nth, int w, size_t elem) {
     return static_cast<size_t>(parent_nth) * 2 * pairs * 64 * elem +

@@ -25,6 +25,17 @@ int main() {
                 CHECK(m2m_smem(got, nph, elem) <= limit || got == 1);
                 if (m2m_smem(rows, nph, elem) <= limit) CHECK(got == rows);
             }
+            // children summed first: fewer rows before the kernel is given up
+            for (int w : {2, 4, 6, 8, 10})
+                for (int cth = 4; cth <= nth; ++cth)
+                    for (int rows : {1, 2, 4, 8, 16, 32, 64}) {
+                        auto fits = [&](int r) {
+                            return m2m_sum_smem(r, cth, nph, 2 * cth, w, elem) + kSmemStatic <= limit;
+                        };
+                        const int got = m2m_sum_fit_rows(rows, cth, nph, 2 * cth, w, elem, limit);
+                        CHECK(got <= rows && (got ? fits(got) : !fits(1)));
+                        if (got && 2 * got <= rows) CHECK(!fits(2 * got));
+                    }
             for (int w : {8, 12, 16, 24, 32})
                 for (int cth = 4; cth <= nth; ++cth) {
                     if (l2l_m_smem(1, nth, cth, w, elem) + kSmemStatic > limit) continue;  // refused at setup
@@ -42,6 +53,9 @@ int main() {
     CHECK(l2l_m_fit_pairs(2, 58, 34, 12, 16, limit) == 1);
     CHECK(m2m_fit_rows(16, 68, 8, limit) == 16);
     CHECK(m2m_fit_rows(16, 68, 16, limit) == 8);
+    // and rows of the summed aggregation
+    CHECK(m2m_sum_fit_rows(64, 45, 158, 90, 6, 8, limit) == 64);
+    CHECK(m2m_sum_fit_rows(64, 45, 158, 90, 6, 16, limit) == 16);
     std::printf(bad ? "%d FAILED\n" : "ALL OK\n", bad);
     return bad != 0;
 }
