@@ -428,6 +428,7 @@ private:
     void build_m2l_items(int max_chunk);
     std::string build_m2l_families(const Plan& plan);
     std::string ensure_graph(int prec, bool tr, bool krylov);
+    bool own_solve_graph(bool krylov) const;
     std::string setup_tc(const Plan& plan);
     std::string build_transl_device(const Level& L, double2* t);
     void far_m2m_tc(int p, int nr, cudaStream_t s);
@@ -481,7 +482,7 @@ private:
     int n_near_quads_ = 0;
     int* near_qslot_ = nullptr;           //   slots of their partials
     int* near_qred_ptr_ = nullptr;        //   and [n + 1]: target t's slots
-    int near_sym_grid_ = 0;               // k_near_sym in products of a mixed operator's solves
+    int near_sym_grid_ = 0;               // k_near_sym in a mixed operator's solves beside k_near_direct in its products
     int m_m2m_rows_fast_ = -1;            // many-rhs M2M grid order (-1: precision default)
     int m_l2l_pairs_ = 0;                 // many-rhs L2L column pairs per block (0: precision default)
     std::vector<int2*> l2l_pairs_;       // per parent level: (parent, child entry)

@@ -164,16 +164,14 @@ DeviceOp::~DeviceOp() {
     if (err_host_) cudaFreeHost(err_host_);
 }
 
-// Persistent blocks of k_near_sym: per_sm per SM, but at least four tiles per
-// block, so that a small operator leaves room for the kernels of others
-// running beside it.
+// Blocks of the near-field kernel that products run: per_sm per SM.
 void DeviceOp::set_near_grid(int per_sm) {
     if (near_kernel_ != 0 && n_near_quads_) {  // k_near_direct: every resident warp of the grid takes quads
         near_grid_ = std::max(1, std::min((n_near_quads_ + kNdThreads / 32 - 1) / (kNdThreads / 32),
                                           std::max(1, per_sm) * sms_));
         return;
     }
-    near_grid_ = std::max(1, std::min(n_near_tiles_ / 4, std::max(1, per_sm) * sms_));
+    near_grid_ = near_sym_blocks(n_near_tiles_, per_sm, sms_);
 }
 
 void launch_wait_runs_out(long long limit, int* status) { k_wait_runs_out<<<1, 32>>>(limit, status); }
@@ -1117,7 +1115,7 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
                 MLFMA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&near_direct_occ_, k_near_direct, kNdThreads, 0));
                 near_direct_occ_ = std::max(1, near_direct_occ_);
                 near_kernel_ = n_near_quads_ ? 2 : 0;
-                near_sym_grid_ = std::max(1, std::min(n_near_tiles_ / 4, near_occ_ * sms_));
+                near_sym_grid_ = near_sym_blocks(n_near_tiles_, near_occ_, sms_);
                 near_per_sm_ = near_kernel_ ? near_direct_occ_ : near_occ_;
                 set_near_grid(near_per_sm_);
                 DevNearBlock* d_nb = upload(nb);
@@ -1472,13 +1470,13 @@ void DeviceOp::run_near(const double2* xt, cudaStream_t s, bool krylov) {
         cudaMemsetAsync(ynear_, 0, sizeof(double2) * n_, s);
         return;
     }
-    const bool ordered = krylov && precision_ != kFp64;
-    const bool quads = near_kernel_ && n_near_quads_ && !ordered;
+    const bool quads = near_runs_quads(near_kernel_ != 0, n_near_quads_ > 0, krylov, precision_ != kFp64);
     if (quads)
         k_near_direct<<<near_grid_, kNdThreads, 0, s>>>(near_quads_, n_near_quads_, near_bz_, xt, near_qslot_,
                                                          near_part_);
     else
-        k_near_sym<<<ordered ? near_sym_grid_ : near_grid_, kSymThreads, kSymSmemBytes, s>>>(
+        // (near_grid_ is k_near_sym's unless this is the solve that differs)
+        k_near_sym<<<own_solve_graph(krylov) ? near_sym_grid_ : near_grid_, kSymThreads, kSymSmemBytes, s>>>(
             near_tiles_, n_near_tiles_, near_bz_, xt, near_slot_, near_part_, err_dev_);
     k_near_reduce<<<blocks_for(static_cast<long long>(n_) * kReduceLanes, 256), 256, 0, s>>>(
         quads ? near_qred_ptr_ : near_red_ptr_, near_part_, n_, ynear_);
@@ -1504,8 +1502,12 @@ void DeviceOp::enqueue_core(cudaStream_t s, int prec, bool tr, bool krylov) {
     cudaStreamWaitEvent(s, ev_join_, 0);
 }
 
+bool DeviceOp::own_solve_graph(bool krylov) const {
+    return krylov && near_solve_differs(near_kernel_ != 0, n_near_quads_ > 0, precision_ != kFp64);
+}
+
 std::string DeviceOp::ensure_graph(int prec, bool tr, bool krylov) {
-    const int t = tr ? 1 : 0, k = krylov && precision_ != kFp64 ? 1 : 0;
+    const int t = tr ? 1 : 0, k = own_solve_graph(krylov) ? 1 : 0;
     if (graph_exec_[prec][t][k] || !use_graph_) return {};
     cudaGraph_t& g = graph_[prec][t][k];
     cudaGetLastError();  // an earlier caller's error is not this capture's
@@ -1525,7 +1527,7 @@ std::string DeviceOp::ensure_graph(int prec, bool tr, bool krylov) {
 }
 
 void DeviceOp::launch_core(cudaStream_t s, int prec, bool tr, bool krylov) {
-    const int t = tr ? 1 : 0, k = krylov && precision_ != kFp64 ? 1 : 0;
+    const int t = tr ? 1 : 0, k = own_solve_graph(krylov) ? 1 : 0;
     if (graph_exec_[prec][t][k]) cudaGraphLaunch(graph_exec_[prec][t][k], s); else enqueue_core(s, prec, tr, krylov);
 }
 
@@ -2519,7 +2521,7 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
         // near field: persistent blocks per SM, timed on the whole product (it
         // runs beside the far-field chain and competes with it for the SMs)
         if (n_near_tiles_) {
-            float bt = 1e30f;
+            float bt = 1e30f, bsym = 1e30f;
             int bk = near_per_sm_, bkind = near_kernel_;
             for (int kind : n_near_quads_ ? std::vector<int>{0, 2} : std::vector<int>{0})
                 for (int k = 1; k <= (kind ? near_direct_occ_ : near_occ_); ++k) {
@@ -2527,6 +2529,7 @@ std::string DeviceOp::autotune(int nr, int reps, TuneReport* rep) {
                     set_near_grid(k);
                     const float t = timed(product);
                     if (t < bt) { bt = t; bk = k; bkind = kind; }
+                    if (!kind && t < bsym) { bsym = t; near_sym_grid_ = near_grid_; }  // (a mixed operator's solves)
                 }
             near_kernel_ = bkind;
             near_per_sm_ = bk;

@@ -14,6 +14,21 @@ namespace mlfma {
 // aggregation, whose stencils are static, has its own bound at setup).
 constexpr size_t kSmemStatic = 1024;
 
+// Near field of one product.  Blocks of k_near_sym: per_sm per SM, but at least
+// four tiles each, so that a small operator leaves room for the kernels beside it.
+inline int near_sym_blocks(int tiles, int per_sm, int sms) {
+    return std::max(1, std::min(tiles / 4, std::max(1, per_sm) * sms));
+}
+// Which kernel a product runs: k_near_direct where it is chosen and there are quads,
+// except in a mixed operator's solves, which keep the order of k_near_sym's sums.
+inline bool near_runs_quads(bool chosen, bool quads, bool solve, bool mixed) {
+    return chosen && quads && !(solve && mixed);
+}
+// Whether a solve's product differs from the operator's own and has its own graph.
+inline bool near_solve_differs(bool chosen, bool quads, bool mixed) {
+    return near_runs_quads(chosen, quads, false, mixed) != near_runs_quads(chosen, quads, true, mixed);
+}
+
 // Aggregation child by child (k_m2m): up to eight children's theta passes.
 // elem: bytes of a complex value.
 inline size_t m2m_smem(int rows, int child_nph, size_t elem) {

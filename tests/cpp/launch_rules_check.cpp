@@ -13,7 +13,25 @@ static int bad = 0;
         if (!(c) && bad++ < 20) std::printf("line %d: %s\n", __LINE__, #c); \
     } while (0)
 
+// The near field's kernel and graph: a solve has its own only where a mixed
+// operator's products run quads, so that one chosen grid serves both elsewhere.
+static void near_rules() {
+    for (bool chosen : {false, true})
+        for (bool quads : {false, true})
+            for (bool mixed : {false, true}) {
+                CHECK(near_runs_quads(chosen, quads, false, mixed) == (chosen && quads));
+                CHECK(near_runs_quads(chosen, quads, true, mixed) == (chosen && quads && !mixed));
+                CHECK(near_solve_differs(chosen, quads, mixed) == (chosen && quads && mixed));
+            }
+    for (int tiles : {1, 3, 4, 1000, 100000})
+        for (int per_sm : {0, 1, 5}) {
+            const int b = near_sym_blocks(tiles, per_sm, 148);
+            CHECK(b >= 1 && b <= 148 * (per_sm ? per_sm : 1) && (b == 1 || 4 * b <= tiles));
+        }
+}
+
 int main() {
+    near_rules();
     const size_t limit = 232448;  // opt-in shared memory of a block
     for (size_t elem : {8u, 16u})
         for (int nth = 4; nth <= 160; ++nth) {
