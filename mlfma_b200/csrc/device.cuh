@@ -428,6 +428,7 @@ private:
     void build_m2l_items(int max_chunk);
     std::string build_m2l_families(const Plan& plan);
     std::string ensure_graph(int prec, bool tr, bool krylov);
+    std::string capture_graph(int prec, bool tr, bool krylov);
     bool own_solve_graph(bool krylov) const;
     std::string setup_tc(const Plan& plan);
     std::string build_transl_device(const Level& L, double2* t);

@@ -1169,6 +1169,7 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
         MLFMA_CK(cudaStreamSynchronize(stream_));
         MLFMA_CK(cudaStreamSynchronize(cudaStreamLegacy));  // the memsets above run there
         MLFMA_CK(cudaGetLastError());
+        if (own_solve_graph(true)) capture_graph(precision_, false, true);  // (without it: plain launches)
         ready_ = true;
         return {};
     } catch (const std::exception& e) {
@@ -1506,9 +1507,20 @@ bool DeviceOp::own_solve_graph(bool krylov) const {
     return krylov && near_solve_differs(near_kernel_ != 0, n_near_quads_ > 0, precision_ != kFp64);
 }
 
+// Where a solve's product differs, a forward one is captured at setup already (and,
+// after a change of launch shapes, with the next product): a solve that may not
+// allocate (mlfma_gmres_noalloc) launches what is there, and plain launches cost it
+// 113 in place of 101 us a step (1,920 unknowns, complex float).
 std::string DeviceOp::ensure_graph(int prec, bool tr, bool krylov) {
+    if (!use_graph_) return {};
+    const std::string e = capture_graph(prec, tr, krylov);
+    if (e.empty() && !krylov && !tr && prec == precision_ && own_solve_graph(true)) return capture_graph(prec, tr, true);
+    return e;
+}
+
+std::string DeviceOp::capture_graph(int prec, bool tr, bool krylov) {
     const int t = tr ? 1 : 0, k = own_solve_graph(krylov) ? 1 : 0;
-    if (graph_exec_[prec][t][k] || !use_graph_) return {};
+    if (graph_exec_[prec][t][k]) return {};
     cudaGraph_t& g = graph_[prec][t][k];
     cudaGetLastError();  // an earlier caller's error is not this capture's
     MLFMA_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
