@@ -536,17 +536,17 @@ k_m2l_staged(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ item
 //
 // Bound by shared-memory reads (two wavefronts a pair, four a pattern) and
 // instruction issue, so a candidate's transfer rows are staged as shared-memory
-// offsets (a row of zeros where it is not in a target's list 2, about one pair
-// in ten) and the loop is instantiated per number of targets: a shared-memory
-// read and four multiply-adds per pair.  (A source value that is not finite
-// reaches every target anyhow, by a list or through the near field, so the zero
-// rows spread nothing.)  One B200, k_m2l_staged -> this: 8,192 dipoles, level 3
-// (512 boxes, 392 directions) 77 -> 46 us; r = 8 sphere, level 6 (16,344 boxes,
-// 162 directions) 390 -> 204 us, all levels 930 -> 530 us; r = 2 sphere,
-// levels 2-4 22/28/34 -> 20/22/27 us.  In complex float, whose sums keep
-// their order and run in two halves, the same form was issue-bound and no
-// faster (r = 2 sphere 18/19/22 -> 20/26/34 us, r = 8 sphere 498 -> 505 us):
-// complex float keeps k_m2l_staged.
+// offsets (the row past the table where it is not in a target's list 2, about one
+// pair in ten) and the loop is instantiated per number of targets: a shared-memory
+// read and four multiply-adds per pair.  Those of the row past the table are
+// predicated off (at most 1 % of a product, 8,192 dipoles 121.5 -> 122.8 us): a
+// pattern that overflowed may come from a neighbour whose near entries are finite.
+// One B200, k_m2l_staged -> this: 8,192 dipoles, level 3 (512 boxes, 392
+// directions) 77 -> 48 us; r = 8 sphere, level 6 (16,344 boxes, 162 directions)
+// 390 -> 204 us, all levels 930 -> 530 us; r = 2 sphere, levels 3 and 4 27/36 ->
+// 23/26 us.  In complex float, whose sums keep their order and run in two halves,
+// the same form was issue-bound and no faster (r = 2 sphere, levels 2-4 18/19/22 ->
+// 20/26/34 us, r = 8 sphere 498 -> 505 us): complex float keeps k_m2l_staged.
 constexpr int kM2LOffsets = 316;
 constexpr int kM2LDirs = 16;            // directions per block
 constexpr int kM2LRow = kM2LDirs * 16;  // bytes of a row of transfer values
@@ -631,13 +631,14 @@ k_m2l_group(const DevLevelT<double>* __restrict__ lvs, int level, const DevM2LFa
                 for (int u = 0; u < U; ++u) an[u] = Al[ssrc[(i + U + u) & 31] * astride];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int4 o4 = soff[i + u];  // (past the list's end: rows of zeros)
+                    const int4 o4 = soff[i + u];  // (past the list's end: in no target's list)
                     const int o[4] = {o4.x, o4.y, o4.z, o4.w};
                     double2 tv[NT];
 #pragma unroll
                     for (int t = 0; t < NT; ++t) tv[t] = *reinterpret_cast<const double2*>(tl + o[t]);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) acc[t] = cfma(tv[t], a[u], acc[t]);
+                    for (int t = 0; t < NT; ++t)
+                        if (o[t] != kM2LOffsets * kM2LRow) acc[t] = cfma(tv[t], a[u], acc[t]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) a[u] = an[u];
