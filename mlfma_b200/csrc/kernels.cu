@@ -1069,10 +1069,17 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
             for (const NearBlock& b : plan.near_blocks)
                 nb.push_back(DevNearBlock{b.row0, b.nrow, b.col0, b.ncol, b.off,
                                           b.self ? (plan.cfg.self_terms ? 2 : 1) : 0, 0});
+            near_block_entries_ = plan.near_entries;
+            if (!plan.near_tiles.empty()) {  // the entries, while the host lays out the tiles
+                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_));
+                DevNearBlock* d_nb = upload(nb);
+                k_near_blocks_assemble<<<blocks_for(near_block_entries_, 128), 128, 0, stream_>>>(
+                    d_nb, static_cast<int>(nb.size()), near_block_entries_, S, near_bz_);
+                MLFMA_CK(cudaGetLastError());
+            }
             std::vector<DevNearTile> nt;
             for (const NearTile& t : plan.near_tiles)
                 nt.push_back(DevNearTile{t.z, t.r0, t.c0, t.i0, t.ni, t.j0, t.nj, t.ld, t.kind, t.slot, t.mode});
-            near_block_entries_ = plan.near_entries;
             n_near_tiles_ = static_cast<int>(nt.size());
             if (n_near_tiles_ > 0) {
                 near_tiles_ = upload(nt);
@@ -1103,7 +1110,6 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
                     n_near_quads_ = static_cast<int>(quads.size() / 4);
                     near_quads_ = upload(quads);
                 }
-                near_bz_ = alloc<double2>(static_cast<size_t>(near_block_entries_));
                 near_part_ = alloc<double2>(parts);
                 near_red_ptr_ = upload(plan.near_red_ptr);
                 near_slot_ = upload(plan.near_slot);
@@ -1118,10 +1124,6 @@ std::string DeviceOp::setup(const Plan& plan, int device, int precision, int max
                 near_sym_grid_ = near_sym_blocks(n_near_tiles_, near_occ_, sms_);
                 near_per_sm_ = near_kernel_ ? near_direct_occ_ : near_occ_;
                 set_near_grid(near_per_sm_);
-                DevNearBlock* d_nb = upload(nb);
-                k_near_blocks_assemble<<<blocks_for(near_block_entries_, 128), 128, 0, stream_>>>(
-                    d_nb, static_cast<int>(nb.size()), near_block_entries_, S, near_bz_);
-                MLFMA_CK(cudaGetLastError());
             }
         }
         // leaves of the block-Jacobi preconditioner (built on first use)
