@@ -29,7 +29,8 @@ solution, on 64 seeded rows against the dense FP64 operator (every
 interaction evaluated directly on the GPU, mlfma_dense_rows).
 
 `--impl reference` times the reference's own CPU code (oracle/_ref, built from
-its sources, single-threaded by construction) on the same workload.
+its sources, single-threaded by construction) on the same workload; where that
+library is not built the line says `unavailable` instead.
 """
 from __future__ import annotations
 
@@ -147,6 +148,15 @@ def parity_vector(n):
     """The seeded input vector of the reference arm's products (and of the GPU
     arm's parity check against them)."""
     return np.random.default_rng(7).standard_normal(n) + 1j * np.random.default_rng(8).standard_normal(n)
+
+
+NO_REFERENCE = "the reference's library (oracle/_ref) is not built: its sources are not on this machine"
+
+
+def reference_available() -> bool:
+    sys.path.insert(0, HERE)
+    from oracle import ref_lib
+    return ref_lib.available()
 
 
 def run_reference(steps: int, warmup: int, save_y: str | None = None) -> dict:
@@ -839,6 +849,9 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return 0
+        if not reference_available():
+            print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
+            return 0
         r = run_reference(args.steps, max(args.warmup, 0), save_y=args.save_y)
         line = {"metric": METRIC, "value": r["value"], "unit": UNIT, "impl": "reference", "n_gpus": args.gpus,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": r["ms_per_step"],
@@ -865,7 +878,7 @@ def main():
     # CPU baseline in a child process (rank 0, N = 1), overlapping GPU setup.
     cpu_proc = None
     ref_y = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and reference_available():
         fd, ref_y = tempfile.mkstemp(suffix=".npz")
         os.close(fd)
         cpu_proc = subprocess.Popen([sys.executable, os.path.abspath(__file__), "--impl", "reference",
@@ -898,6 +911,8 @@ def main():
                                  f"{r['config'].get('reference_setup_s', 0):.0f} s setup"}
             except Exception as e:  # noqa: BLE001
                 cpu = {"value": None, "unit": UNIT, "cores": 1, "kind": "reference", "sample": f"failed: {e}"}
+        elif solo and not args.no_cpu_baseline:
+            cpu = {"value": None, "unit": UNIT, "cores": 1, "kind": "reference", "sample": f"unavailable: {NO_REFERENCE}"}
         parity = None
         if ref_y is not None:
             try:
