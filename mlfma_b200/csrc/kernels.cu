@@ -269,13 +269,16 @@ void DeviceOp::build_m2l_items(int max_chunk) {
 // A warp's task is a family and a run of directions.  With four targets per
 // family a pattern load serves about three pairs, but a level of few boxes then
 // leaves most warps of the GPU without a task, so families shrink to two targets
-// or one until there are kM2LMinTasksPerSM per SM (the r = 1.13 sphere's 56-box
-// level with 392 directions: families of four 20 us, of one 16 us).  A level of
-// fewer than kM2LMinPairDirs (pair, direction)s gets no families and keeps
-// k_m2l_staged: filling the blocks' transfer values (81 KB each) is then most of
-// the work, and the large blocks queue behind the near field's (600 dipoles,
-// 2.0M: whole product 44.4 us staged, 45.4 us by families; a 512-box level of
-// 8,192 dipoles, 21M: product 181 and 150 us).
+// or one until there are kM2LMinTasksPerSM per SM (56 boxes with 392 directions,
+// families tried below the line: of four 20 us, of one 16 us).
+//
+// A level of fewer than kM2LMinPairDirs (pair, direction)s gets no families and
+// keeps k_m2l_staged: there filling the blocks' transfer values (81 KB each) is most
+// of the work.  Level times, k_m2l_staged and families: above the line 3.2M 25.9 and
+// 19.3 us, 3.6M 21.4 and 18.8, 4.1M 20.5 and 20.4, 7.1M 27.0 and 22.9, 16M 59.0 and
+// 44.5; below it 1.1M 18.4 and 14.3, 2.5M 20.6 and 18.9, 2.7M (600 dipoles) 20.5
+// and 18.4.  So the line is on the safe side: nothing above it is slower, and the
+// smallest operators keep k_m2l_staged's sums to the last bit.
 std::string DeviceOp::build_m2l_families(const Plan& plan) {
     std::vector<DevM2LFamily> fams;
     std::vector<short> off;

@@ -543,7 +543,7 @@ k_m2l_staged(const DevLevelT<R>* __restrict__ lvs, const int4* __restrict__ item
 // pattern that overflowed may come from a neighbour whose near entries are finite.
 // One B200, k_m2l_staged -> this: 8,192 dipoles, level 3 (512 boxes, 392
 // directions) 77 -> 48 us; r = 8 sphere, level 6 (16,344 boxes, 162 directions)
-// 390 -> 204 us, all levels 930 -> 530 us; r = 2 sphere, levels 3 and 4 27/36 ->
+// 392 -> 220 us, all levels 932 -> 566 us; r = 2 sphere, levels 3 and 4 27/36 ->
 // 23/26 us.  In complex float, whose sums keep their order and run in two halves,
 // the same form was issue-bound and no faster (r = 2 sphere, levels 2-4 18/19/22 ->
 // 20/26/34 us, r = 8 sphere 498 -> 505 us): complex float keeps k_m2l_staged.

@@ -139,10 +139,15 @@ struct NearTile {
 // of at most kNearQuadCols columns, applied four to a warp (k_near_direct); a
 // larger one keeps k_near_sym's alone.  The narrow tiles write more partial sums,
 // which cost little while they stay in the L2 (about 0.08 per entry: 36M entries
-// 46 MB; 133M entries 170 MB).  One B200, whole products, k_near_sym and
-// k_near_direct: 7.8M entries 197 and 184 us FP64, 133 and 112 us complex-float
-// far field; 36M entries 511 and 486 us (complex float); 133M entries 2,008 and
-// 2,080 us.
+// 46 MB; 133M entries 170 MB).  One B200, spheres, whole products, k_near_sym and
+// k_near_direct (us; complex-float far field in brackets): 7.8M entries 183 and 173
+// (121, 105); 36M 697 and 695 (471, 450); 44M 722 and 720 (492, 471); 50M in leaves
+// of up to 20 sources 4,102 and 3,607 (2,996, 2,470); 52M, up to 120, 757 and 763
+// (521, 504); 70M, up to 30, 3,945 and 3,517 (2,858, 2,407); 125M, up to 200, 1,300
+// and 1,136 (916, 737); 133M, up to 54 2,848 and
+// 2,956 (1,820, 1,910).  Above the line it depends on how full the leaves' tiles
+// are, which the number of entries does not tell; the large fields stay with
+// k_near_sym, which their solves run in any case.
 constexpr int kNearQuadCols = 32;
 constexpr long long kNearQuadEntries = 48ll << 20;
 struct NearTiling {
